@@ -158,6 +158,7 @@ tms_status tms_destroy(tms_ctx* ctx)
   fr(ctx->lxxlo.n);
   fr(ctx->cgm_x);
   fr(ctx->cgm_ps);
+  fr(ctx->cgm_r);
   fr(ctx->cgm);
   if (ctx->cgm_h) cudaFreeHost(ctx->cgm_h);
   fr(ctx->xlo32.d);

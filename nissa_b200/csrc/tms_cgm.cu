@@ -80,6 +80,73 @@ namespace
   // iteration count (the reference's final_iter).
   size_t per_site_bytes(int prec) { return prec == PREC_F64 ? 192 : prec == PREC_F32 ? 96 : 52; }
 
+  // iterations whose shift updates are applied together: the largest divisor of
+  // the replay length up to CGM_MAX_WINDOW (a replay starts and ends a window)
+  int cgm_window(int graph_iters)
+  {
+    int w = std::min(graph_iters, CGM_MAX_WINDOW);
+    while (graph_iters % w) w--;
+    return w;
+  }
+
+  // the residuals of a window besides the running one, as many as memory has room
+  // for: a window of `want` iterations, or of a divisor of it
+  tms_status ensure_window(tms_ctx* ctx, int prec, size_t fbytes, int want)
+  {
+    if (ctx->cgm_window && ctx->cgm_window_prec == prec && ctx->cgm_window_want == want) return TMS_OK;
+    TRY(drop_graph(ctx, 6));
+    TRY(drop_graph(ctx, 7));
+    if (ctx->cgm_r) cudaFree(ctx->cgm_r);
+    ctx->cgm_r = nullptr;
+    ctx->cgm_window = 0;
+    // what the rest of the call may still allocate (the e/o solver's FP64 and inner
+    // fields, the staging buffer) stays free
+    const size_t reserve = (size_t)32 * 192 * ctx->g.stride;
+    int w = want;
+    for (; w > 1; w--)
+      {
+        if (want % w) continue;
+        size_t avail = 0, total = 0;
+        CU(cudaMemGetInfo(&avail, &total));
+        if (avail < fbytes * (w - 1) + reserve) continue;
+        if (cudaMalloc(&ctx->cgm_r, fbytes * (w - 1)) == cudaSuccess) break;
+        ctx->cgm_r = nullptr;
+        cudaGetLastError(); // out of memory: a shorter window
+      }
+    ctx->cgm_window = w;
+    ctx->cgm_window_prec = prec;
+    ctx->cgm_window_want = want;
+    return TMS_OK;
+  }
+
+  template <int W, class V, class R, class Get>
+  void cgm_flush_w(tms_ctx* ctx, cudaStream_t s, const Get& get, int64_t words)
+  {
+    CgmWindow<W, V> win;
+    for (int w = 0; w < W; w++) win.r[w] = get(w);
+    cgm_flush_kernel<W, V, R><<<div_up(words, CGM_FLUSH_THREADS), CGM_FLUSH_THREADS, 0, s>>>(
+      words, win, (V*)ctx->cgm_x, (V*)ctx->cgm_ps, words, ctx->cgm);
+  }
+
+  // the shift updates of the W iterations since the last flush
+  template <class V, class R, class Get>
+  void cgm_flush(tms_ctx* ctx, cudaStream_t s, int W, const Get& get, int64_t words)
+  {
+    ctx->launches += 2;
+    switch (W)
+      {
+      case 8: cgm_flush_w<8, V, R>(ctx, s, get, words); break;
+      case 7: cgm_flush_w<7, V, R>(ctx, s, get, words); break;
+      case 6: cgm_flush_w<6, V, R>(ctx, s, get, words); break;
+      case 5: cgm_flush_w<5, V, R>(ctx, s, get, words); break;
+      case 4: cgm_flush_w<4, V, R>(ctx, s, get, words); break;
+      case 3: cgm_flush_w<3, V, R>(ctx, s, get, words); break;
+      case 2: cgm_flush_w<2, V, R>(ctx, s, get, words); break;
+      default: cgm_flush_w<1, V, R>(ctx, s, get, words);
+      }
+    cgm_flushed_kernel<<<1, 1, 0, s>>>(ctx->cgm);
+  }
+
   template <int P, int LF>
   tms_status cgm_run(tms_ctx* ctx, const LinkT<LF>& U, int nshift, const double* sigma, const double* target,
                      int niter, double b2, int* iters, float* ms)
@@ -116,6 +183,14 @@ namespace
     const Field& r = hi ? ctx->lx64[2] : ctx->lxlo[1];
     const Field& p = hi ? ctx->lx64[3] : ctx->lxlo[2];
     const Field& t = hi ? ctx->lx64[4] : ctx->lxlo[3];
+    TRY(ensure_window(ctx, P, fbytes, cgm_window(ctx->graph_iters)));
+    // the window's residuals: iteration j of a window writes R(j), reading its predecessor's
+    const int W = ctx->cgm_window;
+    auto R = [&](int j) {
+      Field f = r;
+      if (j < W - 1) f.d = (unsigned char*)ctx->cgm_r + fbytes * j;
+      return f;
+    };
     // solution / direction views of shift k
     auto shift_field = [&](void* base, int k) {
       Field f;
@@ -150,23 +225,23 @@ namespace
       }
     CU(cudaMemcpyAsync(ctx->cgm, &S, sizeof S, cudaMemcpyHostToDevice, ctx->stream));
     const OpParams* prm = ctx->prm + 1; // the CGM operator: mu = 0
-    const size_t shift_elems = fbytes / (P == PREC_F64 ? sizeof(double2) : P == PREC_F32 ? sizeof(float4) : sizeof(uint4));
+    using Word = typename std::conditional<P == PREC_F64, double2, float4>::type;
+    const int64_t words = (int64_t)(fbytes / sizeof(Word));
     TRY(capture(ctx, slot, [&](cudaStream_t cs) {
       auto V = [](const Field& f, int par) { return view_par<P>(f, par); };
       const int* stop = &ctx->cgm->stop;
       for (int it = 0; it < ctx->graph_iters; it++)
         {
-          ++ctx->launches;
-          cgm_begin_kernel<<<1, 1, 0, cs>>>(ctx->cgm);
+          const int j = it % W;
+          const Field rin = R((j + W - 1) % W), rout = R(j);
           EpiTmQ<P, true> a{{V(t, 0), V(t, 1)}, {V(p, 0), V(p, 1)}, prm, +1.0};
           launch_hop_v<P, LF>(ctx, cs, 0, 2, V(p, 0), V(p, 1), U, prm, a, FinCgm1{ctx->cgm}, stop);
-          EpiCgm2<P> b{{V(t, 0), V(t, 1)}, {V(r, 0), V(r, 1)}, prm, ctx->cgm};
-          launch_hop_v<P, LF>(ctx, cs, 0, 2, V(t, 0), V(t, 1), U, prm, b, FinCgm2{ctx->cgm}, stop);
+          EpiCgm2<P> b{{V(t, 0), V(t, 1)}, {V(rin, 0), V(rin, 1)}, {V(rout, 0), V(rout, 1)}, prm, ctx->cgm};
+          launch_hop_v<P, LF>(ctx, cs, 0, 2, V(t, 0), V(t, 1), U, prm, b, FinCgm2{ctx->cgm, j}, stop);
           ++ctx->launches;
-          cgm_update_kernel<P><<<div_up(n, 256), 256, 0, cs>>>(n, view<P>(r), view<P>(p),
-                                                               view<P>(shift_field(ctx->cgm_x, 0)),
-                                                               view<P>(shift_field(ctx->cgm_ps, 0)), shift_elems,
-                                                               ctx->cgm);
+          cgm_p_kernel<P><<<div_up(n, 256), 256, 0, cs>>>(n, view<P>(rout), view<P>(p), ctx->cgm);
+          if (j == W - 1)
+            cgm_flush<Word, typename SpinorT<P>::R>(ctx, cs, W, [&](int w) { return (const Word*)R(w).d; }, words);
         }
     }));
     CU(cudaEventRecord(ctx->ev0, ctx->stream));

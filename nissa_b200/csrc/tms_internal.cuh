@@ -115,6 +115,8 @@ struct tms_ctx
   void* cgm_x = nullptr;
   void* cgm_ps = nullptr;
   int cgm_prec = -1, cgm_nshift = 0;
+  void* cgm_r = nullptr; // residuals of a window of iterations besides the running one
+  int cgm_window = 0, cgm_window_prec = -1, cgm_window_want = 0;
 
   // lx spinor buffers on the device for the propagator entry points (tms_prop.cu)
   double* lxbuf[2] = {nullptr, nullptr};

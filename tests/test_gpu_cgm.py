@@ -74,3 +74,28 @@ def test_cgm_argument_errors(cuda_device):
         with pytest.raises(TmError) as e:
             lat.inv_tmQ2_cgm(0.16, [0.01, 0.1], src, 3, 1e-24)
         assert e.value.status == 1
+
+
+@pytest.mark.parametrize("graph_iters", [2, 5, 6, 7, 8, 24])
+@pytest.mark.parametrize("precision,niter", [("double", 100000), ("double", 13), ("single", 100000)])
+def test_cgm_window_lengths(cuda_device, graph_iters, precision, niter):
+    """Shift updates applied by windows of 2 to 8 iterations, with shifts that stop inside a window and with a
+    solve cut inside one (13 iterations), against one iteration at a time (windows of 1, replays of 11)."""
+    T, L = 6, 4
+    masses = [0.01, 0.05, 0.3]
+    res = [1e-20, 1e-18, 1e-14]
+    src = wl.random_spinor(T * L ** 3, 45)
+    with Lattice(T, L) as lat:
+        lat.upload_conf(wl.gauge_conf(T, L, 0.35, seed=46))
+        got = []
+        for n in (11, graph_iters):
+            lat.set_tuning("graph_iters", n)
+            got.append(lat.inv_tmQ2_cgm(0.16, masses, src, niter, res, precision=precision, raise_on_error=False))
+        for k in range(3):
+            assert got[0][1][k]["iterations"] == got[1][1][k]["iterations"]
+            # FP64: the same operations per site in the same order, up to their contraction into FMAs.  FP32: two
+            # solutions within their residues, |dx| <= 2 |A^-1| |r|, so 2 sqrt(res) cond(A) of |x|; here
+            # A = Q_W^2 + m^2 has eigenvalues between m^2 and (1/2k + 4)^2, and a tenth of that bound is asked for
+            cond = (0.5 / 0.16 + 4) ** 2 / masses[k] ** 2
+            tol = 1e-12 if precision == "double" else 0.2 * np.sqrt(res[k]) * min(cond, 1e3)
+            assert rel(got[1][0][k], got[0][0][k]) < tol, k
