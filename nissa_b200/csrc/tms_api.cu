@@ -271,32 +271,28 @@ tms_status tms_hop_eo(tms_ctx* ctx, int par_out, const double* in, double* out, 
 {
   TRY(check_conf(ctx));
   if (par_out != 0 && par_out != 1) return fail(ctx, TMS_ERR_BAD_ARG, "parity must be 0 or 1");
-  TRY(set_params(ctx, 1.0, 0.0, has_anis, anis));
-  Field &a = ctx->f64[6], &b = ctx->f64[7];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  EpiPlain<PREC_F64> e{{view<PREC_F64>(b), view<PREC_F64>(b)}};
-  launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, par_out, 1, a, a, links64(ctx), ctx->prm, e);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
+  OpBuffers b;
+  TRY(op_begin(ctx, in, out, bytes, b));
+  const OpParams prm{1.0, 0.0, has_anis ? anis : 1.0};
+  launch_hop_aos<false>(ctx, par_out, b.in, prm, EpiPlain<PREC_A64>{{view_aos(b.out), view_aos(b.out)}});
+  return op_end(ctx, b, out, bytes);
 }
 
 static tms_status diag_common(tms_ctx* ctx, double kappa, double mu, const double* in, double* out, int inverse)
 {
   if (!ctx) return TMS_ERR_BAD_ARG;
   CU(cudaSetDevice(ctx->device));
-  TRY(set_params(ctx, kappa, mu, 0, 1.0));
-  Field &a = ctx->f64[6], &b = ctx->f64[7];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  const int n = (int)ctx->g.Vh;
+  TRY(check_params(ctx, kappa, mu));
+  const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
+  OpBuffers b;
+  TRY(op_begin(ctx, in, out, bytes, b));
+  const int64_t n = ctx->g.Vh * 12;
   ++ctx->launches;
-  diag_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, view<PREC_F64>(a), view<PREC_F64>(b), ctx->prm,
-                                                                   1.0, inverse);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  diag_aos_kernel<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, reinterpret_cast<const double2*>(b.in),
+                                                           reinterpret_cast<double2*>(b.out), OpParams{kappa, mu, 1.0},
+                                                           inverse);
+  return op_end(ctx, b, out, bytes);
 }
 
 tms_status tms_tmDee(tms_ctx* ctx, double kappa, double mu, const double* in, double* out)
@@ -309,88 +305,90 @@ tms_status tms_inv_tmDee(tms_ctx* ctx, double kappa, double mu, const double* in
   return diag_common(ctx, kappa, mu, in, out, 1);
 }
 
+// out = K(sgn mu) in, or K(+mu) K(-mu) in (odd -> odd)
+static tms_status kern_common(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in, double* out,
+                              bool square)
+{
+  TRY(check_conf(ctx));
+  TRY(check_params(ctx, kappa, mu));
+  const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
+  Field &te = ctx->f64[5], &t1 = ctx->f64[4];
+  TRY(alloc_field(ctx, te, PREC_F64));
+  if (square) TRY(alloc_field(ctx, t1, PREC_F64));
+  OpBuffers b;
+  TRY(op_begin(ctx, in, out, bytes, b));
+  const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
+  if (ctx->g.Vh > AOS_KERN_SITES)
+    {
+      Field &x = ctx->f64[6], &y = ctx->f64[7];
+      TRY(alloc_field(ctx, x, PREC_F64));
+      TRY(alloc_field(ctx, y, PREC_F64));
+      TRY(put_params(ctx, prm));
+      launch_aos_split(ctx, b.in, x);
+      if (square) kern_op<PREC_F64>(ctx, links64(ctx), x, te, t1, -1.0, ctx->prm);
+      kern_op<PREC_F64>(ctx, links64(ctx), square ? t1 : x, te, y, +1.0, ctx->prm);
+      launch_aos_join(ctx, y, b.out);
+      return op_end(ctx, b, out, bytes);
+    }
+  auto kern = [&](const double* x, double* y, double sgn) {
+    double* t = (double*)te.d;
+    launch_hop_aos<false>(ctx, 0, x, prm, EpiInvDiag<PREC_A64>{{view_aos(t), view_aos(t)}, nullptr, sgn});
+    launch_hop_aos<false>(ctx, 1, t, prm,
+                          EpiKern<PREC_A64, false>{{view_aos(y), view_aos(y)}, {view_aos(x), view_aos(x)}, nullptr, sgn});
+  };
+  if (square) kern(b.in, (double*)t1.d, -1.0);
+  kern(square ? (double*)t1.d : b.in, b.out, +1.0);
+  return op_end(ctx, b, out, bytes);
+}
+
 tms_status tms_kern_eoprec(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in,
                            double* out)
 {
-  TRY(check_conf(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
-  Field &a = ctx->f64[6], &b = ctx->f64[7], &te = ctx->f64[5];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  TRY(alloc_field(ctx, te, PREC_F64));
-  kern_op<PREC_F64>(ctx, links64(ctx), a, te, b, +1.0, ctx->prm);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  return kern_common(ctx, kappa, has_anis, anis, mu, in, out, false);
 }
 
 tms_status tms_kern_eoprec_square(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in,
                                   double* out)
 {
-  TRY(check_conf(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
-  Field &a = ctx->f64[6], &b = ctx->f64[7], &te = ctx->f64[5], &t1 = ctx->f64[4];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  TRY(alloc_field(ctx, te, PREC_F64));
-  TRY(alloc_field(ctx, t1, PREC_F64));
-  kern_op<PREC_F64>(ctx, links64(ctx), a, te, t1, -1.0, ctx->prm);
-  kern_op<PREC_F64>(ctx, links64(ctx), t1, te, b, +1.0, ctx->prm);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  return kern_common(ctx, kappa, has_anis, anis, mu, in, out, true);
 }
 
-// full-lattice operators: lx spinors are split into the two parities of
-// fields 6 (even) / 7 (odd) -> outputs in 4 (even) / 5 (odd)
+// full-lattice operators: out = Q(+mu) in, or Q(-mu) Q(+mu) in
 static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in,
                              double* out, bool square)
 {
   TRY(check_conf(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
-  Field* f = ctx->f64;
-  for (int i = 1; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
-  const int64_t Vh = ctx->g.Vh;
-  // in: split lx -> (e, o)
-  const double* src = in;
+  TRY(check_params(ctx, kappa, mu));
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
-  if (ctx->ptr_mode == TMS_PTR_HOST)
+  const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
+  OpBuffers b;
+  if (!square || ctx->g.V <= AOS_Q2_SITES)
     {
-      TRY(ensure_stage(ctx, bytes));
-      CU(cudaMemcpyAsync(ctx->stage, in, bytes, cudaMemcpyHostToDevice, ctx->stream));
-      src = ctx->stage;
+      Field& temp = ctx->lx64[6];
+      if (square) TRY(alloc_field(ctx, temp, PREC_F64, 2 * ctx->g.stride));
+      TRY(op_begin(ctx, in, out, bytes, b));
+      auto q = [&](const double* x, double* y, double sgn) {
+        launch_hop_aos<true>(ctx, 0, x, prm,
+                             EpiTmQ<PREC_A64, false>{{view_aos(y), view_aos(y)}, {view_aos(x), view_aos(x)}, nullptr, sgn});
+      };
+      q(b.in, square ? (double*)temp.d : b.out, +1.0);
+      if (square) q((double*)temp.d, b.out, -1.0);
+      return op_end(ctx, b, out, bytes);
     }
-  const int n = (int)Vh;
-  ++ctx->launches;
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo, view<PREC_F64>(f[6]));
-  ++ctx->launches;
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo + Vh,
-                                                                       view<PREC_F64>(f[7]));
-  auto U = links64(ctx);
-  auto V = [&](int i) { return view<PREC_F64>(f[i]); };
-  if (!square)
-    {
-      EpiTmQ<PREC_F64, false> e{{V(4), V(5)}, {V(6), V(7)}, ctx->prm, +1.0};
-      launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, 0, 2, f[6], f[7], U, ctx->prm, e);
-    }
-  else
-    {
-      // temp = Q(+mu) in ; out = Q(-mu) temp
-      EpiTmQ<PREC_F64, false> e1{{V(2), V(3)}, {V(6), V(7)}, ctx->prm, +1.0};
-      launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, 0, 2, f[6], f[7], U, ctx->prm, e1);
-      EpiTmQ<PREC_F64, false> e2{{V(4), V(5)}, {V(2), V(3)}, ctx->prm, -1.0};
-      launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, 0, 2, f[2], f[3], U, ctx->prm, e2);
-    }
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, f[4], ctx->lx_of_eo, ctx->g.V, out, false));
-  // second parity goes to the same staging/destination buffer
-  double* d = (ctx->ptr_mode == TMS_PTR_HOST) ? ctx->stage : out;
-  ++ctx->launches;
-  soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(5), ctx->lx_of_eo + Vh, d);
-  CU(cudaGetLastError());
-  if (ctx->ptr_mode == TMS_PTR_HOST)
-    CU(cudaMemcpyAsync(out, ctx->stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  return finish(ctx);
+  Field* f = ctx->f64;
+  for (int i = 2; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
+  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(put_params(ctx, prm));
+  launch_lx_split(ctx, b.in, f[6], f[7]);
+  auto q = [&](int x, int y, double sgn) {
+    EpiTmQ<PREC_F64, false> e{{view<PREC_F64>(f[y]), view<PREC_F64>(f[y + 1])},
+                              {view<PREC_F64>(f[x]), view<PREC_F64>(f[x + 1])}, ctx->prm, sgn};
+    launch_hop<PREC_F64>(ctx, ctx->stream, 0, 2, f[x], f[x + 1], links64(ctx), ctx->prm, e);
+  };
+  q(6, 2, +1.0);
+  q(2, 4, -1.0);
+  launch_lx_paste(ctx, f[4], f[5], b.out);
+  return op_end(ctx, b, out, bytes);
 }
 
 tms_status tms_apply_tmQ(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in,

@@ -376,55 +376,79 @@ tms_status tms_inv_tmclovDee(tms_ctx* ctx, double kappa, double mu, int dag, con
   return finish(ctx);
 }
 
+// out = K_clov(dag) in, or K_clov(false) K_clov(true) in (odd -> odd), in the caller's layout
+static tms_status clov_kern_common(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, int dag, const double* in,
+                                   double* out, bool square)
+{
+  TRY(check_clover(ctx));
+  TRY(check_params(ctx, kappa, mu));
+  TRY(ensure_clover_inverse(ctx, kappa, mu));
+  const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
+  Field &te = ctx->f64[5], &t1 = ctx->f64[4];
+  TRY(alloc_field(ctx, te, PREC_F64));
+  if (square) TRY(alloc_field(ctx, t1, PREC_F64));
+  OpBuffers b;
+  TRY(op_begin(ctx, in, out, bytes, b));
+  const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
+  if (ctx->g.Vh > AOS_CLOVER_SITES)
+    {
+      Field &x = ctx->f64[6], &y = ctx->f64[7];
+      TRY(alloc_field(ctx, x, PREC_F64));
+      TRY(alloc_field(ctx, y, PREC_F64));
+      TRY(put_params(ctx, prm));
+      launch_aos_split(ctx, b.in, x);
+      if (square) clov_kern_op<PREC_F64>(ctx, links64(ctx), clov64(ctx), x, te, t1, 1, ctx->prm);
+      clov_kern_op<PREC_F64>(ctx, links64(ctx), clov64(ctx), square ? t1 : x, te, y, square ? 0 : dag, ctx->prm);
+      launch_aos_join(ctx, y, b.out);
+      return op_end(ctx, b, out, bytes);
+    }
+  const ClovT<PREC_A64> cl{ctx->cl64, ctx->icl64, (int)ctx->g.Vh};
+  auto kern = [&](const double* x, double* y, int dg) {
+    double* t = (double*)te.d;
+    launch_hop_aos<false>(ctx, 0, x, prm, EpiInvClov<PREC_A64>{{view_aos(t), view_aos(t)}, cl, dg});
+    launch_hop_aos<false>(ctx, 1, t, prm,
+                          EpiClovKern<PREC_A64, false>{{view_aos(y), view_aos(y)}, {view_aos(x), view_aos(x)}, cl, nullptr, dg});
+  };
+  if (square) kern(b.in, (double*)t1.d, 1);
+  kern(square ? (double*)t1.d : b.in, b.out, square ? 0 : dag);
+  return op_end(ctx, b, out, bytes);
+}
+
 tms_status tms_tmclovDkern_eoprec(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, int dag,
                                   const double* in, double* out)
 {
-  TRY(check_clover(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
-  TRY(ensure_clover_inverse(ctx, kappa, mu));
-  Field &a = ctx->f64[6], &b = ctx->f64[7], &te = ctx->f64[5];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  TRY(alloc_field(ctx, te, PREC_F64));
-  clov_kern_op<PREC_F64>(ctx, links64(ctx), clov64(ctx), a, te, b, dag, ctx->prm);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  return clov_kern_common(ctx, kappa, has_anis, anis, mu, dag, in, out, false);
 }
 
 tms_status tms_tmclovDkern_eoprec_square(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu,
                                          const double* in, double* out)
 {
-  TRY(check_clover(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
-  TRY(ensure_clover_inverse(ctx, kappa, mu));
-  Field &a = ctx->f64[6], &b = ctx->f64[7], &te = ctx->f64[5], &t1 = ctx->f64[4];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
-  TRY(alloc_field(ctx, b, PREC_F64));
-  TRY(alloc_field(ctx, te, PREC_F64));
-  TRY(alloc_field(ctx, t1, PREC_F64));
-  clov_kern_op<PREC_F64>(ctx, links64(ctx), clov64(ctx), a, te, t1, 1, ctx->prm);
-  clov_kern_op<PREC_F64>(ctx, links64(ctx), clov64(ctx), t1, te, b, 0, ctx->prm);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
-  return finish(ctx);
+  return clov_kern_common(ctx, kappa, has_anis, anis, mu, 0, in, out, true);
 }
 
 tms_status tms_apply_tmclovQ(tms_ctx* ctx, double kappa, int has_anis, double anis, double mu, const double* in,
                              double* out)
 {
   TRY(check_clover(ctx));
-  TRY(set_params(ctx, kappa, mu, has_anis, anis));
+  TRY(check_params(ctx, kappa, mu));
+  const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
+  OpBuffers b;
+  TRY(op_begin(ctx, in, out, bytes, b));
+  const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
+  if (ctx->g.V <= AOS_CLOVER_SITES)
+    {
+      const ClovT<PREC_A64> cl{ctx->cl64, ctx->icl64, (int)ctx->g.Vh};
+      launch_hop_aos<true>(ctx, 0, b.in, prm,
+                           EpiTmClovQ<PREC_A64>{{view_aos(b.out), view_aos(b.out)}, {view_aos(b.in), view_aos(b.in)}, cl, nullptr});
+      return op_end(ctx, b, out, bytes);
+    }
   Field* f = ctx->f64;
   for (int i = 4; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
-  const int64_t Vh = ctx->g.Vh;
-  TRY(spinor_in(ctx, in, ctx->lx_of_eo, ctx->g.V, f[6]));
-  TRY(spinor_in(ctx, in, ctx->lx_of_eo + Vh, ctx->g.V, f[7]));
+  TRY(put_params(ctx, prm));
+  launch_lx_split(ctx, b.in, f[6], f[7]);
   tmclovQ_op(ctx, f[6], f[7], f[4], f[5], ctx->prm);
-  CU(cudaGetLastError());
-  TRY(spinor_out(ctx, f[4], ctx->lx_of_eo, ctx->g.V, out, false));
-  TRY(spinor_out(ctx, f[5], ctx->lx_of_eo + Vh, ctx->g.V, out, true));
-  return finish(ctx);
+  launch_lx_paste(ctx, f[4], f[5], b.out);
+  return op_end(ctx, b, out, bytes);
 }
 
 } // extern "C"

@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "tms_kernels.cuh"
+#include "tms_hop_aos.cuh"
 
 namespace tms
 {
@@ -28,7 +29,7 @@ namespace tms
   struct ClovT
   {
     using R = typename SpinorT<P>::R;
-    using V2 = typename std::conditional<P == PREC_F64, double2, float2>::type;
+    using V2 = typename std::conditional<P == PREC_F64 || P == PREC_A64, double2, float2>::type;
     const V2* __restrict__ cl;  // [par][36][Vh]
     const V2* __restrict__ icl; // [72][Vh], even sites
     int Vh;
@@ -88,6 +89,43 @@ namespace tms
       apply_block(par, 1, site, C<R>{kcf, -m}, in, o);
     }
 
+    // component c of (z + block) in, z the twisted diagonal of c's chirality
+    template <class V>
+    __device__ __forceinline__ C<R> block_comp(int par, int site, int c, C<R> z, const V* in) const
+    {
+      const int b = c / 6, a = c % 3;
+      const bool low = c % 6 >= 3;
+      const V* i0 = in + 6 * b;
+      const V* i1 = i0 + 3;
+      C<R> o = cmul(z, C<R>{in[c].x, in[c].y});
+#pragma unroll
+      for (int e = 0; e < 3; e++)
+        {
+          // upper: c0 i0 + c1^+ i1; lower: c1 i0 - c0 i1
+          const C<R> c0 = cl_elem(par, (2 * b) * 9 + 3 * a + e, site);
+          const C<R> c1 = cl_elem(par, (2 * b + 1) * 9 + (low ? 3 * a + e : 3 * e + a), site);
+          const C<R> x0 = {i0[e].x, i0[e].y}, x1 = {i1[e].x, i1[e].y};
+          o = low ? cadd(csub(o, cmul(c0, x1)), cmul(c1, x0)) : cadd(cadd(o, cmul(c0, x0)), cjmul(c1, x1));
+        }
+      return o;
+    }
+    // component c of T_ee^-1(dag) in
+    template <class V>
+    __device__ __forceinline__ C<R> inv_comp(int site, bool dag, int c, const V* in) const
+    {
+      const int b = c / 6, r = c % 6;
+      const bool stored = b == (dag ? 1 : 0);
+      C<R> s = {R(0), R(0)};
+#pragma unroll
+      for (int e = 0; e < 6; e++)
+        {
+          C<R> m = icl_elem(b * 36 + (stored ? r * 6 + e : e * 6 + r), site);
+          if (!stored) m.im = -m.im;
+          s = cadd(s, cmul(m, C<R>{in[6 * b + e].x, in[6 * b + e].y}));
+        }
+      return s;
+    }
+
     // inv_tmclovDee_or_oo_eos (dirac_operator_tmclovD_eoprec.hpp:24-44) on an even site:
     // the chirality `high` (0, or 1 when dag) takes the stored inverse, the other its conjugate
     __device__ __forceinline__ void inv(int site, bool dag, const C<R> in[12], C<R> o[12]) const
@@ -125,6 +163,12 @@ namespace tms
       pick(out[0], out[1], p).store(ieo, o);
       return 0.0;
     }
+    // component c from the site's hop (the operand x, where there is one, likewise)
+    template <class V>
+    __device__ __forceinline__ C<typename SpinorT<P>::R> comp(int, int ieo, int c, const V* acc, const V*) const
+    {
+      return cl.inv_comp(ieo, dag != 0, c, acc);
+    }
   };
 
   // out = g5 ( T_oo(dag) x - hop/4 ): tmclovDkern_eoprec_eos
@@ -154,6 +198,15 @@ namespace tms
         }
       pick(out[0], out[1], p).store(ieo, acc);
       return n2;
+    }
+    template <class V>
+    __device__ __forceinline__ C<typename SpinorT<P>::R> comp(int p, int ieo, int c, const V* acc, const V* xv) const
+    {
+      using R = typename SpinorT<P>::R;
+      const R m = (dag != 0) == (c < 6) ? -R(prm->mu) : R(prm->mu);
+      const C<R> d = cl.block_comp(p, ieo, c, C<R>{R(1.0 / (2.0 * prm->kappa)), m}, xv);
+      const C<R> q = cscale(C<R>{acc[c].x, acc[c].y}, R(0.25));
+      return (c < 6) ? csub(d, q) : csub(q, d);
     }
   };
 
@@ -272,6 +325,15 @@ namespace tms
         }
       pick(out[0], out[1], p).store(ieo, acc);
       return 0.0;
+    }
+    template <class V>
+    __device__ __forceinline__ C<typename SpinorT<P>::R> comp(int p, int ieo, int c, const V* acc, const V* xv) const
+    {
+      using R = typename SpinorT<P>::R;
+      const R kcf = R(1.0 / (2.0 * prm->kappa)), m = R(prm->mu);
+      const C<R> v = {xv[c].x, xv[c].y}, d = cl.block_comp(p, ieo, c, C<R>{R(0), R(0)}, xv);
+      const C<R> im = {-m * v.im, m * v.re}, h = cscale(C<R>{acc[c].x, acc[c].y}, R(0.5)), k = cscale(v, kcf);
+      return (c < 6) ? cadd(cadd(d, csub(k, h)), im) : cadd(csub(csub(h, k), d), im);
     }
   };
 }

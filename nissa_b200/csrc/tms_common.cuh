@@ -32,7 +32,7 @@
 
 namespace tms
 {
-  enum Prec { PREC_F64 = 0, PREC_F32 = 1, PREC_F16 = 2 };
+  enum Prec { PREC_F64 = 0, PREC_F32 = 1, PREC_F16 = 2, PREC_A64 = 3 }; // A64: FP64 in the caller's layout (tms_hop_aos.cuh)
   enum LinkFmt { LINK_F64_18 = 0, LINK_F32_12 = 1, LINK_F32_18 = 2, LINK_I16_12 = 3, LINK_F64_12 = 4, LINK_H16_12 = 5 };
 
   // ------------------------------------------------------------- geometry
@@ -66,10 +66,10 @@ namespace tms
     return s;
   }
 
-  // e/o index of the forward / backward neighbour in direction mu (0=t,1=x,2=y,3=z)
+  // lx index of the forward / backward neighbour in direction mu (0=t,1=x,2=y,3=z)
   // and whether the hop crosses the time boundary
   template <int MU>
-  __device__ __forceinline__ int nbr_up(const Lattice& g, const Site& s, bool& wrap_t)
+  __device__ __forceinline__ int nbr_up_lx(const Lattice& g, const Site& s, bool& wrap_t)
   {
     int lx;
     wrap_t = false;
@@ -82,11 +82,11 @@ namespace tms
         wrap_t = (s.t == g.T - 1);
         lx = wrap_t ? s.lx - (g.T - 1) * st : s.lx + st;
       }
-    return lx >> 1;
+    return lx;
   }
 
   template <int MU>
-  __device__ __forceinline__ int nbr_dw(const Lattice& g, const Site& s, bool& wrap_t)
+  __device__ __forceinline__ int nbr_dw_lx(const Lattice& g, const Site& s, bool& wrap_t)
   {
     int lx;
     wrap_t = false;
@@ -99,7 +99,20 @@ namespace tms
         wrap_t = (s.t == 0);
         lx = wrap_t ? s.lx + (g.T - 1) * st : s.lx - st;
       }
-    return lx >> 1;
+    return lx;
+  }
+
+  // their e/o indices
+  template <int MU>
+  __device__ __forceinline__ int nbr_up(const Lattice& g, const Site& s, bool& wrap_t)
+  {
+    return nbr_up_lx<MU>(g, s, wrap_t) >> 1;
+  }
+
+  template <int MU>
+  __device__ __forceinline__ int nbr_dw(const Lattice& g, const Site& s, bool& wrap_t)
+  {
+    return nbr_dw_lx<MU>(g, s, wrap_t) >> 1;
   }
 
   // ---------------------------------------- programmatic dependent launch

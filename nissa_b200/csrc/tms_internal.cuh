@@ -7,6 +7,7 @@
 #include "tms_pipe.cuh"
 #include "tms_hop_sp.cuh"
 #include "tms_hop_tma.cuh"
+#include "tms_hop_aos.cuh"
 #include "tms_clover.cuh"
 
 #include <cmath>
@@ -268,13 +269,25 @@ namespace tms_int
     return TMS_OK;
   }
 
-  inline tms_status set_params(tms_ctx* ctx, double kappa, double mu, int has_anis, double anis, int slot = 0)
+  inline tms_status check_params(tms_ctx* ctx, double kappa, double mu)
   {
     if (!(kappa > 0.0) || !std::isfinite(kappa) || !std::isfinite(mu))
       return fail(ctx, TMS_ERR_BAD_ARG, "invalid kappa %g / mu %g", kappa, mu);
-    OpParams h{kappa, mu, has_anis ? anis : 1.0};
+    return TMS_OK;
+  }
+
+  inline tms_status put_params(tms_ctx* ctx, const OpParams& h, int slot = 0)
+  {
     return put_small(ctx, ctx->prm + slot, &h, sizeof h);
   }
+
+  inline tms_status set_params(tms_ctx* ctx, double kappa, double mu, int has_anis, double anis, int slot = 0)
+  {
+    TRY(check_params(ctx, kappa, mu));
+    return put_params(ctx, OpParams{kappa, mu, has_anis ? anis : 1.0}, slot);
+  }
+
+  inline LinkT<LINK_F64_18> links64(tms_ctx* c) { return LinkT<LINK_F64_18>{c->U64, (int)c->g.Vh}; }
 
   // ------------------------------------------------------------ hop launch
   // a launch with programmatic stream serialisation (when enabled): the kernel
@@ -311,17 +324,17 @@ namespace tms_int
         auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
         static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         (void)attr;
-        launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm, epi,
+        launch_pdl(c, k, npar * div_up(c->g.Vh, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm, epi,
                    reducer(c), fin, stop);
         return;
       }
     else
       {
-    if constexpr (P != PREC_F64)
+        if constexpr (P != PREC_F64)
           {
             if (c->hop_cfg[P] == 5)
               {
-                launch_pdl(c, hop_sp_kernel<P, LF, Epi, Fin>, div_up(nsite, HOP_SP_THREADS), HOP_SP_THREADS, 0, s, c->g,
+                launch_pdl(c, hop_sp_kernel<P, LF, Epi, Fin>, npar * div_up(c->g.Vh, HOP_SP_THREADS), HOP_SP_THREADS, 0, s, c->g,
                            par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
                 return;
               }
@@ -335,7 +348,7 @@ namespace tms_int
                 auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
                 static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
                 (void)attr;
-                launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm,
+                launch_pdl(c, k, npar * div_up(c->g.Vh, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm,
                            epi, reducer(c), fin, stop);
                 return;
               }
@@ -382,15 +395,15 @@ namespace tms_int
         switch (c->hop_cfg[P])
           {
           case 1:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 1>, div_up(nsite, HopCfg<P, 1>::NT), HopCfg<P, 1>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 1>, npar * div_up(c->g.Vh, HopCfg<P, 1>::NT), HopCfg<P, 1>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
             break;
           case 2:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 2>, div_up(nsite, HopCfg<P, 2>::NT), HopCfg<P, 2>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 2>, npar * div_up(c->g.Vh, HopCfg<P, 2>::NT), HopCfg<P, 2>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
             break;
           default:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 0>, div_up(nsite, HopCfg<P, 0>::NT), HopCfg<P, 0>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 0>, npar * div_up(c->g.Vh, HopCfg<P, 0>::NT), HopCfg<P, 0>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
           }
       }
@@ -404,7 +417,6 @@ namespace tms_int
     launch_hop_v<P, LF>(c, s, par_out, npar, view<P>(in_e), view<P>(in_o), U, prm, epi, fin, stop);
   }
 
-  inline LinkT<LINK_F64_18> links64(tms_ctx* c) { return LinkT<LINK_F64_18>{c->U64, (int)c->g.Vh}; }
   inline LinkT<LINK_F64_12> links64r(tms_ctx* c) { return LinkT<LINK_F64_12>{c->U64, (int)c->g.Vh}; }
   // the FP64 residual recomputations of the mixed solvers may read the links as
   // 12 reals when the conf is SU(3) to FP64 rounding
@@ -413,6 +425,100 @@ namespace tms_int
   inline LinkT<LINK_F32_18> links32f(tms_ctx* c) { return LinkT<LINK_F32_18>{c->U32f, (int)c->g.Vh}; }
   inline LinkT<LINK_I16_12> links16r(tms_ctx* c) { return LinkT<LINK_I16_12>{c->U16r, (int)c->g.Vh}; }
   inline LinkT<LINK_H16_12> links16h(tms_ctx* c) { return LinkT<LINK_H16_12>{c->U16h, (int)c->g.Vh}; }
+
+  // ------------------------------------------- operators in the caller's layout
+  // Output sites per hop up to which an operator of several hops works on the
+  // caller's arrays directly; the others convert to planes and back around hops
+  // on planes.  (A single hop, tms_hop_eo or tms_apply_tmQ, is direct at every
+  // size: 32^3x64 hop 424 us, 440 with the conversions.)  Whole calls, direct /
+  // on planes: K^2 at 8400 sites 63.9 / 71.2 us, 20736 72.2 / 79.4, 36864
+  // 91.2 / 87.4, 331776 547 / 459; twisted-clover K^2 at 4096 45.7 / 67.5, 8400
+  // 68.6 / 73.2, 20736 84.5 / 81.8.  The directions' products are spread over a
+  // block, so nothing of a neighbour is reused through L1, which costs the more
+  // the more sites there are to hide latencies.
+  constexpr int64_t AOS_KERN_SITES = 25000, AOS_Q2_SITES = 60000, AOS_CLOVER_SITES = 10000;
+
+  // one hop from `in` to epi.out, both in the caller's layout: e/o order of
+  // parity par_out, or (FULL) lx order; the parameters travel with the launch
+  template <bool FULL, class Epi>
+  void launch_hop_aos(tms_ctx* c, int par_out, const double* in, const OpParams& prm, const Epi& epi)
+  {
+    auto k = hop_aos_dp_kernel<Epi, FULL>;
+    static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, AOS_DP_SMEM);
+    (void)attr;
+    ++c->launches;
+    launch_pdl(c, k, div_up(FULL ? c->g.V : c->g.Vh, HOP_DP_SITES), HOP_DP_THREADS, AOS_DP_SMEM, c->stream, c->g, par_out,
+               reinterpret_cast<const double2*>(in), links64(c), prm, epi);
+  }
+
+  inline SpinorT<PREC_A64> view_aos(const double* p)
+  {
+    return SpinorT<PREC_A64>{reinterpret_cast<double2*>(const_cast<double*>(p)), nullptr, 0};
+  }
+
+  // the caller's layout (device) <-> planes: an e/o spinor, an lx spinor's
+  // parities.  Ordinary launches: overlapped with the hops (programmatic launch),
+  // their shared memory keeps the SMs from returning it to L1, and each hop of
+  // the chain after them runs at half its speed (24^3x48: 160 instead of 86 us).
+  inline void launch_aos_split(tms_ctx* c, const double* in, const Field& f)
+  {
+    ++c->launches;
+    aos_split_kernel<<<div_up(c->g.Vh, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>((int)c->g.Vh, in,
+                                                                                        view<PREC_F64>(f));
+  }
+  inline void launch_aos_join(tms_ctx* c, const Field& f, double* out)
+  {
+    ++c->launches;
+    aos_join_kernel<<<div_up(c->g.Vh, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>((int)c->g.Vh, view<PREC_F64>(f),
+                                                                                       out);
+  }
+  inline void launch_lx_split(tms_ctx* c, const double* in, const Field& ev, const Field& od)
+  {
+    ++c->launches;
+    lx_split_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(
+      c->g, in, view<PREC_F64>(ev), view<PREC_F64>(od));
+  }
+  inline void launch_lx_paste(tms_ctx* c, const Field& ev, const Field& od, double* out)
+  {
+    ++c->launches;
+    lx_paste_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(
+      c->g, view<PREC_F64>(ev), view<PREC_F64>(od), out);
+  }
+
+  // The buffers of one operator call: the caller's own where the kernels can
+  // work on them, else (host pointers, pointers off a 16-byte boundary, an input
+  // that overlaps the output) copies in the staging buffer.
+  struct OpBuffers
+  {
+    const double* in = nullptr;
+    double* out = nullptr;
+  };
+  inline tms_status op_begin(tms_ctx* ctx, const double* in, double* out, size_t bytes, OpBuffers& b)
+  {
+    const bool host = ctx->ptr_mode == TMS_PTR_HOST;
+    if (!host && (!in || !out)) return fail(ctx, TMS_ERR_BAD_ARG, "null spinor");
+    const uintptr_t i = (uintptr_t)in, o = (uintptr_t)out;
+    const bool copy_in = host || i % 16 || (i < o + bytes && o < i + bytes);
+    const bool copy_out = host || o % 16;
+    if (copy_in || copy_out) TRY(ensure_stage(ctx, 2 * bytes));
+    b.in = in;
+    b.out = copy_out ? ctx->stage + bytes / sizeof(double) : out;
+    if (copy_in)
+      {
+        CU(cudaMemcpyAsync(ctx->stage, in, bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream));
+        b.in = ctx->stage;
+      }
+    return TMS_OK;
+  }
+  inline tms_status op_end(tms_ctx* ctx, const OpBuffers& b, double* out, size_t bytes)
+  {
+    CU(cudaGetLastError());
+    if (b.out != out)
+      CU(cudaMemcpyAsync(out, b.out, bytes, ctx->ptr_mode == TMS_PTR_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice,
+                         ctx->stream));
+    CU(cudaStreamSynchronize(ctx->stream));
+    return TMS_OK;
+  }
 
   // --------------------------------------------------------- conf kernels
   static __global__ void conf_to_soa_kernel(Lattice g, const double* __restrict__ src, int layout, int unfold,
@@ -572,6 +678,17 @@ namespace tms_int
 #pragma unroll
     for (int c = 0; c < 12; c++) v[c] = diag_apply(v[c], z, c);
     out.store(i, v);
+  }
+
+  // the same on the caller's layout, a complex component per thread (in == out allowed)
+  static __global__ void diag_aos_kernel(int64_t n, const double2* in, double2* out, OpParams prm, int inverse)
+  {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const C<double> z = inverse ? zinvdiag<double>(prm, 1.0) : zdiag<double>(prm, 1.0);
+    const double2 w = in[i];
+    const C<double> v = diag_apply(C<double>{w.x, w.y}, z, (int)(i % 12));
+    out[i] = make_double2(v.re, v.im);
   }
 
   // ------------------------------------------------------ spinor transfer

@@ -248,6 +248,8 @@ namespace tms
   // ------------------------------------------------------------ epilogues
   // Each epilogue consumes the accumulated hop of one site (parity p, index
   // ieo) and returns its contribution to the kernel's reduction (if any).
+  // pre() and comp() are the same for one component c of the site, for the hop
+  // on the caller's layout: pre() the factors that do not depend on the site.
 
   // (FP32 arithmetic: the factors in FP32, from correctly rounded reciprocals,
   // instead of FP64 divisions in every thread)
@@ -279,6 +281,20 @@ namespace tms
     return (c < 6) ? cmul(v, z) : cmul(v, cconj(z));
   }
 
+  __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+  __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+  __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+  __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+  // diag_apply with the component a run-time value, contracted as the compiler
+  // contracts it for a constant one, so that the results are the same bits
+  template <typename R>
+  __device__ __forceinline__ C<R> diag_comp(C<R> v, C<R> z, int c)
+  {
+    const bool up = c < 6;
+    const R p = mul_rn(v.im, z.im), q = up ? mul_rn(v.im, z.re) : -mul_rn(v.re, z.im);
+    return {fma_rn(v.re, z.re, up ? -p : p), fma_rn(up ? v.re : v.im, up ? z.im : z.re, q)};
+  }
+
   // out = hop (tmn2Deo_or_tmn2Doe_eos)
   template <int P>
   struct EpiPlain
@@ -289,6 +305,12 @@ namespace tms
     {
       pick(out[0], out[1], p).store(ieo, acc);
       return 0.0;
+    }
+    using R = typename SpinorT<P>::R;
+    __device__ __forceinline__ C<R> pre() const { return {}; }
+    __device__ __forceinline__ void comp(int p, int ieo, int c, C<R> acc, C<R>) const
+    {
+      pick(out[0], out[1], p).store1(ieo, c, acc);
     }
   };
 
@@ -308,6 +330,12 @@ namespace tms
       for (int c = 0; c < 12; c++) acc[c] = diag_apply(acc[c], z, c);
       pick(out[0], out[1], p).store(ieo, acc);
       return 0.0;
+    }
+    using R = typename SpinorT<P>::R;
+    __device__ __forceinline__ C<R> pre() const { return zinvdiag<R>(*prm, sgn); }
+    __device__ __forceinline__ void comp(int p, int ieo, int c, C<R> acc, C<R> z) const
+    {
+      pick(out[0], out[1], p).store1(ieo, c, diag_comp(acc, z, c));
     }
   };
 
@@ -346,6 +374,15 @@ namespace tms
         }
       pick(out[0], out[1], p).store(ieo, acc);
       return n2;
+    }
+    using R = typename SpinorT<P>::R;
+    __device__ __forceinline__ C<R> pre() const { return zdiag<R>(*prm, sgn); }
+    __device__ __forceinline__ void comp(int p, int ieo, int c, C<R> acc, C<R> z) const
+    {
+      const C<R> d = diag_comp(pick(x[0], x[1], p).load1(ieo, c), z, c);
+      const C<R> q = cscale(acc, R(0.25));
+      acc = (c < 6) ? csub(d, q) : csub(q, d);
+      pick(out[0], out[1], p).store1(ieo, c, acc);
     }
   };
 
@@ -456,6 +493,15 @@ namespace tms
         }
       pick(out[0], out[1], p).store(ieo, acc);
       return n2;
+    }
+    using R = typename SpinorT<P>::R;
+    __device__ __forceinline__ C<R> pre() const { return {R(1.0 / (2.0 * prm->kappa)), R(sgn * prm->mu)}; }
+    __device__ __forceinline__ void comp(int p, int ieo, int c, C<R> acc, C<R> z) const
+    {
+      const C<R> xv = pick(x[0], x[1], p).load1(ieo, c);
+      const C<R> im = {-z.im * xv.im, z.im * xv.re}, h = cscale(acc, R(0.5)), k = cscale(xv, z.re);
+      acc = (c < 6) ? cadd(csub(k, h), im) : cadd(csub(h, k), im);
+      pick(out[0], out[1], p).store1(ieo, c, acc);
     }
   };
 
@@ -908,14 +954,11 @@ namespace tms
     constexpr int NT = HopCfg<P, CFG>::NT;
     pdl_enter();
     if (stop && *stop) return;
-    const int idx = blockIdx.x * NT + threadIdx.x;
-    int p = par_out, ieo = idx;
-    if (npar == 2)
-      {
-        p = (idx >= g.Vh) ? 1 : 0;
-        ieo = idx - (p ? (int)g.Vh : 0);
-      }
-    const bool active = (idx < npar * g.Vh);
+    // both parities: alternating blocks, so that the two uses of a link (forward
+    // from one parity, backward from the other) meet in L2
+    const int p = (npar == 2) ? blockIdx.x & 1 : par_out;
+    const int ieo = ((npar == 2) ? blockIdx.x >> 1 : blockIdx.x) * NT + threadIdx.x;
+    const bool active = (ieo < g.Vh);
     double part = 0.0;
     if (active)
       {
@@ -1351,6 +1394,46 @@ namespace tms
     const unsigned x = q % (unsigned)g.LX;
     const unsigned t = q / (unsigned)g.LX;
     return (int)((t + x + y + z) & 1u);
+  }
+
+  // an e/o spinor in the caller's layout <-> planes, staged likewise
+  static __global__ void __launch_bounds__(LXCOPY_THREADS)
+    aos_split_kernel(int n, const double* __restrict__ aos, SpinorT<PREC_F64> out)
+  {
+    __shared__ double sh[LXCOPY_THREADS * LXCOPY_PITCH];
+    const int base = blockIdx.x * LXCOPY_THREADS;
+    const int nsite = min(LXCOPY_THREADS, n - base);
+    const double* in = aos + (size_t)base * 24;
+    for (int k = threadIdx.x; k < nsite * 24; k += LXCOPY_THREADS) sh[(k / 24) * LXCOPY_PITCH + k % 24] = in[k];
+    __syncthreads();
+    if ((int)threadIdx.x >= nsite) return;
+    const double* v = sh + threadIdx.x * LXCOPY_PITCH;
+    C<double> c[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) c[k] = {v[2 * k], v[2 * k + 1]};
+    out.store(base + threadIdx.x, c);
+  }
+  static __global__ void __launch_bounds__(LXCOPY_THREADS)
+    aos_join_kernel(int n, SpinorT<PREC_F64> in, double* __restrict__ aos)
+  {
+    __shared__ double sh[LXCOPY_THREADS * LXCOPY_PITCH];
+    const int base = blockIdx.x * LXCOPY_THREADS;
+    const int nsite = min(LXCOPY_THREADS, n - base);
+    if ((int)threadIdx.x < nsite)
+      {
+        C<double> c[12];
+        in.load(base + threadIdx.x, c);
+        double* v = sh + threadIdx.x * LXCOPY_PITCH;
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+          {
+            v[2 * k] = c[k].re;
+            v[2 * k + 1] = c[k].im;
+          }
+      }
+    __syncthreads();
+    double* out = aos + (size_t)base * 24;
+    for (int k = threadIdx.x; k < nsite * 24; k += LXCOPY_THREADS) out[k] = sh[(k / 24) * LXCOPY_PITCH + k % 24];
   }
 
   template <int P>
