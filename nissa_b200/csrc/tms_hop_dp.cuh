@@ -110,4 +110,82 @@ namespace tms
         if (two) dp_accumulate(d, spin, get(d, k + 1), f, acc[1]);
       }
   }
+
+  template <typename R>
+  struct DpShare
+  {
+    C<R> u[8][6][HOP_DP_SITES]; // direction, product (row 0 colours, row 1 colours), site
+  };
+
+  // adds direction D's products times the hop factor f
+  template <int D, typename R>
+  __device__ __forceinline__ void dp_add(const DpShare<R>& sh, int lane, R f, C<R> acc[12])
+  {
+    C<R> u0[3], u1[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      {
+        u0[c] = cscale(sh.u[D][c][lane], f);
+        u1[c] = cscale(sh.u[D][3 + c][lane], f);
+      }
+    reconstruct<D / 2, !(D & 1)>(acc, u0, u1);
+  }
+
+  template <int P, int LF, class Epi, class Fin>
+  __global__ void __launch_bounds__(HOP_DP_THREADS, 2)
+    hop_dp_kernel(Lattice g, int par_out, int npar, SpinorT<P> in_e, SpinorT<P> in_o, LinkT<LF> U, const OpParams* prm,
+                  Epi epi, Reducer red, Fin fin, const int* __restrict__ stop)
+  {
+    using R = typename SpinorT<P>::R;
+    __shared__ DpShare<R> sh;
+    const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
+    const int chunk = (npar == 2) ? blockIdx.x >> 1 : blockIdx.x;
+    const int p = (npar == 2) ? blockIdx.x & 1 : par_out;
+    const bool active = chunk * HOP_DP_SITES + lane < g.Vh;
+    const int ieo = active ? chunk * HOP_DP_SITES + lane : (int)g.Vh - 1;
+    const Site s = eo_site(g, p, ieo);
+    const int n = dp_neighbour(g, s, d) >> 1;
+    C<R> L[9];
+    R ls, ss;
+    U.template load_scaled<false>((d & 1) ? 1 - p : p, d >> 1, (d & 1) ? n : ieo, L, ls);
+    pdl_enter();
+    if (stop && *stop) return; // the same for the whole grid: this kernel writes it after its last block's hop
+    {
+      C<R> v[12], a[3], b[3], u0[3], u1[3];
+      (p ? in_e : in_o).load_raw(n, v, ss);
+      const bool cross = dp_cross(d);
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        {
+          a[c] = {cross ? v[9 + c].re : v[6 + c].re, cross ? v[9 + c].im : v[6 + c].im};
+          b[c] = {cross ? v[6 + c].re : v[9 + c].re, cross ? v[6 + c].im : v[9 + c].im};
+        }
+      dp_products<R>(d, v, v + 3, a, b, L, ss * ls, u0, u1);
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        {
+          sh.u[d][c][lane] = u0[c];
+          sh.u[d][3 + c][lane] = u1[c];
+        }
+    }
+    __syncthreads();
+    double part = 0.0;
+    if (d == 0 && active)
+      {
+        C<R> acc[12];
+#pragma unroll
+        for (int c = 0; c < 12; c++) acc[c] = {R(0), R(0)};
+        const R anis = R(prm->anis);
+        dp_add<0>(sh, lane, (s.t == g.T - 1) ? R(g.bc_t) : R(1), acc);
+        dp_add<1>(sh, lane, (s.t == 0) ? R(g.bc_t) : R(1), acc);
+        dp_add<2>(sh, lane, anis, acc);
+        dp_add<3>(sh, lane, anis, acc);
+        dp_add<4>(sh, lane, anis, acc);
+        dp_add<5>(sh, lane, anis, acc);
+        dp_add<6>(sh, lane, anis, acc);
+        dp_add<7>(sh, lane, anis, acc);
+        part = epi(p, ieo, acc);
+      }
+    if (Epi::kReduce) grid_reduce<HOP_DP_THREADS>(part, red, fin);
+  }
 }
