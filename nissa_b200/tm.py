@@ -23,6 +23,7 @@ lx conf (V, 4, 3, 3, 2), eo conf (2, Vh, 4, 3, 3, 2).
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 
 import numpy as np
@@ -66,7 +67,7 @@ class _Buf:
                 a = np.ascontiguousarray(a, dtype=np.float64)
             self.ptr, self.device = a.ctypes.data, False
             self.keep = a
-        if shape is not None and int(np.prod(shape)) != (a.numel() if _is_torch(a) else a.size):
+        if shape is not None and math.prod(shape) != (a.numel() if _is_torch(a) else a.size):
             raise ValueError("array has %d elements, expected shape %s" % (
                 a.numel() if _is_torch(a) else a.size, tuple(shape)))
 
