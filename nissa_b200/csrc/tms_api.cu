@@ -379,7 +379,7 @@ static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double an
   for (int i = 2; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
   TRY(op_begin(ctx, in, out, bytes, b));
   TRY(put_params(ctx, prm));
-  launch_lx_split(ctx, b.in, f[6], f[7]);
+  launch_lx_split(ctx, b.in, view<PREC_F64>(f[6]), view<PREC_F64>(f[7]));
   auto q = [&](int x, int y, double sgn) {
     EpiTmQ<PREC_F64, false> e{{view<PREC_F64>(f[y]), view<PREC_F64>(f[y + 1])},
                               {view<PREC_F64>(f[x]), view<PREC_F64>(f[x + 1])}, ctx->prm, sgn};
@@ -387,7 +387,7 @@ static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double an
   };
   q(6, 2, +1.0);
   q(2, 4, -1.0);
-  launch_lx_paste(ctx, f[4], f[5], b.out);
+  launch_lx_paste(ctx, view<PREC_F64>(f[4]), view<PREC_F64>(f[5]), b.out);
   return op_end(ctx, b, out, bytes);
 }
 

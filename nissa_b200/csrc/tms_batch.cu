@@ -644,8 +644,7 @@ tms_status tms_batch_submit(tms_batch* b, int slot, const double* src_lx, double
   Field* f = ctx->f64;
   for (int i = 0; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
   for (auto& e : ctx->ex) TRY(alloc_field(ctx, e, PREC_F64));
-  const int64_t Vh = ctx->g.Vh;
-  const int n = (int)Vh;
+  const int n = (int)ctx->g.Vh;
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
   const double* src = src_lx;
   if (ctx->ptr_mode == TMS_PTR_HOST)
@@ -656,9 +655,8 @@ tms_status tms_batch_submit(tms_batch* b, int slot, const double* src_lx, double
     }
   auto V = [](const Field& x) { return view<PREC_F64>(x); };
   const Field ek = one(w->hi[6], slot), vk = one(w->hi[0], slot);
-  ctx->launches += 3;
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo, V(ek));
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo + Vh, V(ctx->ex[1]));
+  launch_lx_split(ctx, src, V(ek), V(ctx->ex[1]));
+  ctx->launches++;
   diag_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(ek), V(f[5]), ctx->prm, 1.0, 1);
   EpiSrcPrep<PREC_F64> sp{{V(vk), V(vk)}, {V(ctx->ex[1]), V(ctx->ex[1])}};
   launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, 1, 1, f[5], f[5], links64(ctx), ctx->prm, sp);
@@ -714,8 +712,6 @@ tms_status tms_batch_collect(tms_batch* b, int slot, double* sol_lx, tms_stats* 
   TRY(set_params(ctx, kappa, mu, b->has_anis, b->anis));
   Field* f = ctx->f64;
   Field* psi = ctx->ex + 2;
-  const int64_t Vh = ctx->g.Vh;
-  const int n = (int)Vh;
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
   auto U = links64(ctx);
   auto V = [](const Field& x) { return view<PREC_F64>(x); };
@@ -727,9 +723,7 @@ tms_status tms_batch_collect(tms_batch* b, int slot, double* sol_lx, tms_stats* 
   double* d = (ctx->ptr_mode == TMS_PTR_HOST) ? ctx->stage : sol_lx;
   if (ctx->ptr_mode == TMS_PTR_HOST) TRY(ensure_stage(ctx, bytes));
   d = (ctx->ptr_mode == TMS_PTR_HOST) ? ctx->stage : sol_lx;
-  ctx->launches += 2;
-  soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(psi[0]), ctx->lx_of_eo, d);
-  soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(psi[1]), ctx->lx_of_eo + Vh, d);
+  launch_lx_paste(ctx, V(psi[0]), V(psi[1]), d);
   CU(cudaGetLastError());
   if (ctx->ptr_mode == TMS_PTR_HOST) CU(cudaMemcpyAsync(sol_lx, ctx->stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   TRY(finish(ctx));

@@ -117,10 +117,10 @@ tms_status tms_cg_eoprec_square(tms_ctx* ctx, double* sol, const double* guess, 
   if (!sol || !src || niter <= 0 || !(residue > 0)) return fail(ctx, TMS_ERR_BAD_ARG, "bad solver arguments");
   TRY(set_params(ctx, kappa, mu, has_anis, anis));
   Field* f = ctx->f64;
-  TRY(spinor_in(ctx, src, nullptr, ctx->g.Vh, f[0]));
-  if (guess) TRY(spinor_in(ctx, guess, nullptr, ctx->g.Vh, f[1]));
+  TRY(spinor_in(ctx, src, f[0]));
+  if (guess) TRY(spinor_in(ctx, guess, f[1]));
   const tms_status st = cg_dispatch<EoOp>(ctx, precision, niter, residue, guess != nullptr, stats);
-  if (st == TMS_OK || st == TMS_ERR_NOT_CONVERGED) TRY(spinor_out(ctx, f[1], nullptr, ctx->g.Vh, sol, true));
+  if (st == TMS_OK || st == TMS_ERR_NOT_CONVERGED) TRY(spinor_out(ctx, f[1], sol));
   TRY(finish(ctx));
   return st;
 }
@@ -150,7 +150,7 @@ namespace
     launch_hop<PREC_F64, LF>(ctx, ctx->stream, 1, 1, f[5], f[5], U, ctx->prm, sp);
     CU(cudaGetLastError());
     // Eq. (9), from the caller's odd-site guess when given
-    if (guess_Koo) TRY(spinor_in(ctx, guess_Koo, nullptr, ctx->g.Vh, f[1]));
+    if (guess_Koo) TRY(spinor_in(ctx, guess_Koo, f[1]));
     const tms_status st = cg_dispatch<EoOp>(ctx, precision, niter, residue, guess_Koo != nullptr, stats);
     if (st != TMS_OK && st != TMS_ERR_NOT_CONVERGED) return st;
     // Eq. (10): psi_o = K(-mu) x ; Eq. (11): psi_e = D_ee^-1 (eta_e + hop(psi_o)/2)

@@ -111,10 +111,10 @@ tms_status tms_cg_tmclov_eoprec_square(tms_ctx* ctx, double* sol, const double* 
   TRY(set_params(ctx, kappa, mu, has_anis, anis));
   TRY(ensure_clover_inverse(ctx, kappa, mu));
   Field* f = ctx->f64;
-  TRY(spinor_in(ctx, src, nullptr, ctx->g.Vh, f[0]));
-  if (guess) TRY(spinor_in(ctx, guess, nullptr, ctx->g.Vh, f[1]));
+  TRY(spinor_in(ctx, src, f[0]));
+  if (guess) TRY(spinor_in(ctx, guess, f[1]));
   const tms_status st = cg_dispatch<ClovOp>(ctx, precision, niter, residue, guess != nullptr, stats);
-  if (st == TMS_OK || st == TMS_ERR_NOT_CONVERGED) TRY(spinor_out(ctx, f[1], nullptr, ctx->g.Vh, sol, true));
+  if (st == TMS_OK || st == TMS_ERR_NOT_CONVERGED) TRY(spinor_out(ctx, f[1], sol));
   TRY(finish(ctx));
   return st;
 }
@@ -134,8 +134,7 @@ tms_status tms_cg_tmclov_eoprec(tms_ctx* ctx, double* sol_lx, const double* src_
   for (int i = 0; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
   Field *eta = ctx->ex, *psi = ctx->ex + 2; // [0] even, [1] odd
   for (auto& e : ctx->ex) TRY(alloc_field(ctx, e, PREC_F64));
-  const int64_t Vh = ctx->g.Vh;
-  const int n = (int)Vh;
+  const int n = (int)ctx->g.Vh;
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
   auto V = [&](const Field& x) { return view<PREC_F64>(x); };
   auto U = links64(ctx);
@@ -146,10 +145,7 @@ tms_status tms_cg_tmclov_eoprec(tms_ctx* ctx, double* sol_lx, const double* src_
       CU(cudaMemcpyAsync(ctx->stage, src_lx, bytes, cudaMemcpyHostToDevice, ctx->stream));
       src = ctx->stage;
     }
-  ++ctx->launches;
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo, V(eta[0]));
-  ++ctx->launches;
-  aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, src, ctx->lx_of_eo + Vh, V(eta[1]));
+  launch_lx_split(ctx, src, V(eta[0]), V(eta[1]));
   // Eq. (8a): te = T_ee^-1 eta_e ; Eq. (8b): varphi = g5 (eta_o + hop(te)/2) -> f0  (:84-90)
   inv_clov_apply(ctx, eta[0], f[5], 0);
   EpiSrcPrep<PREC_F64> sp{{V(f[0]), V(f[0])}, {V(eta[1]), V(eta[1])}};
@@ -164,10 +160,7 @@ tms_status tms_cg_tmclov_eoprec(tms_ctx* ctx, double* sol_lx, const double* src_
   launch_hop<PREC_F64, LINK_F64_18>(ctx, ctx->stream, 0, 1, psi[1], psi[1], U, ctx->prm, rc);
   CU(cudaGetLastError());
   double* d = (ctx->ptr_mode == TMS_PTR_HOST) ? ctx->stage : sol_lx;
-  ++ctx->launches;
-  soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(psi[0]), ctx->lx_of_eo, d);
-  ++ctx->launches;
-  soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, V(psi[1]), ctx->lx_of_eo + Vh, d);
+  launch_lx_paste(ctx, V(psi[0]), V(psi[1]), d);
   CU(cudaGetLastError());
   if (ctx->ptr_mode == TMS_PTR_HOST) CU(cudaMemcpyAsync(sol_lx, ctx->stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   // the residual check of inv_tmclovD_cg_eoprec (:140-175): |g5 Q_clov sol - src|^2 / |src|^2

@@ -351,14 +351,14 @@ tms_status tms_tmclovDee(tms_ctx* ctx, int par, double kappa, double mu, int dag
   if (par != 0 && par != 1) return fail(ctx, TMS_ERR_BAD_ARG, "parity 0 or 1");
   TRY(set_params(ctx, kappa, mu, 0, 1.0));
   Field &a = ctx->f64[6], &b = ctx->f64[7];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
+  TRY(spinor_in(ctx, in, a));
   TRY(alloc_field(ctx, b, PREC_F64));
   const int n = (int)ctx->g.Vh;
   ++ctx->launches;
   clov_diag_kernel<PREC_F64><<<div_up(n, 128), 128, 0, ctx->stream>>>(n, clov64(ctx), par, ctx->prm, dag,
                                                                       view<PREC_F64>(a), view<PREC_F64>(b));
   CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
+  TRY(spinor_out(ctx, b, out));
   return finish(ctx);
 }
 
@@ -368,11 +368,11 @@ tms_status tms_inv_tmclovDee(tms_ctx* ctx, double kappa, double mu, int dag, con
   TRY(set_params(ctx, kappa, mu, 0, 1.0));
   TRY(ensure_clover_inverse(ctx, kappa, mu));
   Field &a = ctx->f64[6], &b = ctx->f64[7];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
+  TRY(spinor_in(ctx, in, a));
   TRY(alloc_field(ctx, b, PREC_F64));
   inv_clov_apply(ctx, a, b, dag);
   CU(cudaGetLastError());
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
+  TRY(spinor_out(ctx, b, out));
   return finish(ctx);
 }
 
@@ -445,9 +445,9 @@ tms_status tms_apply_tmclovQ(tms_ctx* ctx, double kappa, int has_anis, double an
   Field* f = ctx->f64;
   for (int i = 4; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
   TRY(put_params(ctx, prm));
-  launch_lx_split(ctx, b.in, f[6], f[7]);
+  launch_lx_split(ctx, b.in, view<PREC_F64>(f[6]), view<PREC_F64>(f[7]));
   tmclovQ_op(ctx, f[6], f[7], f[4], f[5], ctx->prm);
-  launch_lx_paste(ctx, f[4], f[5], b.out);
+  launch_lx_paste(ctx, view<PREC_F64>(f[4]), view<PREC_F64>(f[5]), b.out);
   return op_end(ctx, b, out, bytes);
 }
 

@@ -488,17 +488,15 @@ namespace tms_int
     aos_join_kernel<<<div_up(c->g.Vh, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>((int)c->g.Vh, view<PREC_F64>(f),
                                                                                        out);
   }
-  inline void launch_lx_split(tms_ctx* c, const double* in, const Field& ev, const Field& od)
+  inline void launch_lx_split(tms_ctx* c, const double* in, const SpinorT<PREC_F64>& ev, const SpinorT<PREC_F64>& od)
   {
     ++c->launches;
-    lx_split_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(
-      c->g, in, view<PREC_F64>(ev), view<PREC_F64>(od));
+    lx_split_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(c->g, in, ev, od);
   }
-  inline void launch_lx_paste(tms_ctx* c, const Field& ev, const Field& od, double* out)
+  inline void launch_lx_paste(tms_ctx* c, const SpinorT<PREC_F64>& ev, const SpinorT<PREC_F64>& od, double* out)
   {
     ++c->launches;
-    lx_paste_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(
-      c->g, view<PREC_F64>(ev), view<PREC_F64>(od), out);
+    lx_paste_kernel<PREC_F64><<<div_up(c->g.V, LXCOPY_THREADS), LXCOPY_THREADS, 0, c->stream>>>(c->g, ev, od, out);
   }
 
   // The buffers of one operator call: the caller's own where the kernels can
@@ -709,39 +707,35 @@ namespace tms_int
 
   // ------------------------------------------------------ spinor transfer
   // bring an e/o spinor (Vh x 24 doubles, host or device) into a FP64 field
-  inline tms_status spinor_in(tms_ctx* ctx, const double* src, const int* site_map, int64_t nrows, Field& f)
+  inline tms_status spinor_in(tms_ctx* ctx, const double* src, Field& f)
   {
     TRY(alloc_field(ctx, f, PREC_F64));
     const double* d = src;
-    const size_t bytes = (size_t)nrows * 24 * sizeof(double);
+    const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
     if (ctx->ptr_mode == TMS_PTR_HOST)
       {
         TRY(ensure_stage(ctx, bytes));
         CU(cudaMemcpyAsync(ctx->stage, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
         d = ctx->stage;
       }
-    const int n = (int)ctx->g.Vh;
-    ++ctx->launches;
-    aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, d, site_map, view<PREC_F64>(f));
+    launch_aos_split(ctx, d, f);
     CU(cudaGetLastError());
     return TMS_OK;
   }
 
-  // write a FP64 field out as Vh rows (optionally scattered through site_map) of 24 doubles
-  inline tms_status spinor_out(tms_ctx* ctx, const Field& f, const int* site_map, int64_t nrows, double* dst, bool flush)
+  // write a FP64 field out as an e/o spinor (Vh x 24 doubles, host or device)
+  inline tms_status spinor_out(tms_ctx* ctx, const Field& f, double* dst)
   {
-    const size_t bytes = (size_t)nrows * 24 * sizeof(double);
+    const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
     double* d = dst;
     if (ctx->ptr_mode == TMS_PTR_HOST)
       {
         TRY(ensure_stage(ctx, bytes));
         d = ctx->stage;
       }
-    const int n = (int)ctx->g.Vh;
-    ++ctx->launches;
-    soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, view<PREC_F64>(f), site_map, d);
+    launch_aos_join(ctx, f, d);
     CU(cudaGetLastError());
-    if (ctx->ptr_mode == TMS_PTR_HOST && flush)
+    if (ctx->ptr_mode == TMS_PTR_HOST)
       {
         CU(cudaMemcpyAsync(dst, ctx->stage, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CU(cudaStreamSynchronize(ctx->stream));
@@ -788,8 +782,6 @@ namespace tms_int
   inline tms_status lx_in(tms_ctx* ctx, const double* src, Field& full)
   {
     TRY(alloc_field(ctx, full, PREC_F64, 2 * ctx->g.stride));
-    const int64_t Vh = ctx->g.Vh;
-    const int n = (int)Vh;
     const double* d = src;
     if (ctx->ptr_mode == TMS_PTR_HOST)
       {
@@ -798,20 +790,13 @@ namespace tms_int
         CU(cudaMemcpyAsync(ctx->stage, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
         d = ctx->stage;
       }
-    for (int p = 0; p < 2; p++)
-      {
-        ++ctx->launches;
-        aos_to_soa_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, d, ctx->lx_of_eo + p * Vh,
-                                                                             view_par<PREC_F64>(full, p));
-      }
+    launch_lx_split(ctx, d, view_par<PREC_F64>(full, 0), view_par<PREC_F64>(full, 1));
     CU(cudaGetLastError());
     return TMS_OK;
   }
 
   inline tms_status lx_out(tms_ctx* ctx, const Field& full, double* dst)
   {
-    const int64_t Vh = ctx->g.Vh;
-    const int n = (int)Vh;
     const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
     double* d = dst;
     if (ctx->ptr_mode == TMS_PTR_HOST)
@@ -819,12 +804,7 @@ namespace tms_int
         TRY(ensure_stage(ctx, bytes));
         d = ctx->stage;
       }
-    for (int p = 0; p < 2; p++)
-      {
-        ++ctx->launches;
-        soa_to_aos_kernel<PREC_F64><<<div_up(n, 256), 256, 0, ctx->stream>>>(n, view_par<PREC_F64>(full, p),
-                                                                             ctx->lx_of_eo + p * Vh, d);
-      }
+    launch_lx_paste(ctx, view_par<PREC_F64>(full, 0), view_par<PREC_F64>(full, 1), d);
     CU(cudaGetLastError());
     if (ctx->ptr_mode == TMS_PTR_HOST)
       {

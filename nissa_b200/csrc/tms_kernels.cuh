@@ -1342,41 +1342,6 @@ namespace tms
   }
 
   // --------------------------------------------------- layout conversion
-  // host-order AoS doubles (site-major, 24 per site) <-> SoA device spinor.
-  // site_map (optional) gives the AoS row of SoA site i (used for lx <-> eo).
-  template <int P>
-  __global__ void aos_to_soa_kernel(int n, const double* __restrict__ aos, const int* __restrict__ site_map,
-                                    SpinorT<P> out)
-  {
-    using R = typename SpinorT<P>::R;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t row = site_map ? (size_t)site_map[i] : (size_t)i;
-    const double* a = aos + row * 24; // 8-byte accesses: the caller's buffer need not be 16-byte aligned
-    C<R> v[12];
-#pragma unroll
-    for (int c = 0; c < 12; c++) v[c] = {R(a[2 * c]), R(a[2 * c + 1])};
-    out.store(i, v);
-  }
-
-  template <int P>
-  __global__ void soa_to_aos_kernel(int n, SpinorT<P> in, const int* __restrict__ site_map, double* __restrict__ aos)
-  {
-    using R = typename SpinorT<P>::R;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t row = site_map ? (size_t)site_map[i] : (size_t)i;
-    C<R> v[12];
-    in.load(i, v);
-    double* a = aos + row * 24;
-#pragma unroll
-    for (int c = 0; c < 12; c++)
-      {
-        a[2 * c] = (double)v[c].re;
-        a[2 * c + 1] = (double)v[c].im;
-      }
-  }
-
   // split_lx_vector_into_eo_parts / paste_eo_parts_into_lx_vector for whole
   // lx spinors: a block takes LXCOPY_THREADS consecutive lx sites, the AoS side
   // moves through shared memory as one contiguous run of doubles (coalesced,

@@ -156,13 +156,13 @@ extern "C" tms_status tms_hop_eo_noalloc(int T, int L, double bc_t, const double
     {
       noalloc_conf_kernel<<<(int)((V + 127) / 128), 128, 0, s>>>(g, conf, layout,
                                                                    (flags & TMS_CONF_BC_INCLUDED) ? 1 : 0, U);
-      aos_to_soa_kernel<PREC_F64><<<(n + 255) / 256, 256, 0, s>>>(n, in, nullptr, sin);
+      aos_split_kernel<<<(n + LXCOPY_THREADS - 1) / LXCOPY_THREADS, LXCOPY_THREADS, 0, s>>>(n, in, sin);
       EpiPlain<PREC_F64> epi{{sout, sout}};
       Reducer red{nullptr, nullptr, nullptr};
       hop_kernel<PREC_F64, LINK_F64_18, EpiPlain<PREC_F64>, NoFin><<<(n + HOP_THREADS - 1) / HOP_THREADS,
                                                                       HOP_THREADS, 0, s>>>(
         g, par_out, 1, sin, sin, LinkT<LINK_F64_18>{U, n}, prm, epi, red, NoFin{}, nullptr);
-      soa_to_aos_kernel<PREC_F64><<<(n + 255) / 256, 256, 0, s>>>(n, sout, nullptr, out);
+      aos_join_kernel<<<(n + LXCOPY_THREADS - 1) / LXCOPY_THREADS, LXCOPY_THREADS, 0, s>>>(n, sout, out);
       e = cudaGetLastError();
     }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -226,7 +226,7 @@ tms_status tms_slab_pack(tms_ctx* ctx, int par_in, const double* in, double* fac
   if ((par_in != 0 && par_in != 1) || !in || !face_fwd || !face_bwd)
     return fail(ctx, TMS_ERR_BAD_ARG, "bad slab pack arguments");
   Field& a = ctx->f64[6];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
+  TRY(spinor_in(ctx, in, a));
   const int face = face_sites(ctx->g);
   const size_t bytes = (size_t)face * 6 * sizeof(double2);
   double2* d = nullptr;
@@ -254,11 +254,11 @@ tms_status tms_slab_hop(tms_ctx* ctx, int par_out, const double* in, const doubl
     return fail(ctx, TMS_ERR_BAD_ARG, "bad slab hop arguments");
   TRY(set_params(ctx, 1.0, 0.0, has_anis, anis));
   Field &a = ctx->f64[6], &b = ctx->f64[7];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
+  TRY(spinor_in(ctx, in, a));
   TRY(alloc_field(ctx, b, PREC_F64));
   EpiPlain<PREC_F64> e{{view<PREC_F64>(b), view<PREC_F64>(b)}};
   TRY(slab_hop_common(ctx, par_out, in, ghost_fwd, ghost_bwd, a, e));
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
+  TRY(spinor_out(ctx, b, out));
   return finish(ctx);
 }
 
@@ -271,7 +271,7 @@ tms_status tms_slab_kern_half(tms_ctx* ctx, int which, double kappa, double mu, 
     return fail(ctx, TMS_ERR_BAD_ARG, "bad slab operator arguments");
   TRY(set_params(ctx, kappa, mu, has_anis, anis));
   Field &a = ctx->f64[6], &b = ctx->f64[7], &xf = ctx->f64[5];
-  TRY(spinor_in(ctx, in, nullptr, ctx->g.Vh, a));
+  TRY(spinor_in(ctx, in, a));
   TRY(alloc_field(ctx, b, PREC_F64));
   if (which == 0)
     {
@@ -282,12 +282,12 @@ tms_status tms_slab_kern_half(tms_ctx* ctx, int which, double kappa, double mu, 
   else
     {
       // odd output: g5 ((1/2k + i mu g5) x - D_oe in / 4) (the second half, with the gamma5 combine)
-      TRY(spinor_in(ctx, x, nullptr, ctx->g.Vh, xf));
+      TRY(spinor_in(ctx, x, xf));
       EpiKern<PREC_F64, false> e{{view<PREC_F64>(b), view<PREC_F64>(b)}, {view<PREC_F64>(xf), view<PREC_F64>(xf)},
                                  ctx->prm, 1.0};
       TRY(slab_hop_common(ctx, 1, in, ghost_fwd, ghost_bwd, a, e));
     }
-  TRY(spinor_out(ctx, b, nullptr, ctx->g.Vh, out, true));
+  TRY(spinor_out(ctx, b, out));
   return finish(ctx);
 }
 
