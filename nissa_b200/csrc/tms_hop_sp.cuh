@@ -207,9 +207,14 @@ namespace tms
   {
     pdl_enter();
     if (stop && *stop) return;
-    const int p = (npar == 2) ? blockIdx.x & 1 : par_out; // both parities: alternating blocks, as in hop_kernel
-    const int ieo = ((npar == 2) ? blockIdx.x >> 1 : blockIdx.x) * HOP_SP_THREADS + threadIdx.x;
-    const bool active = (ieo < g.Vh);
+    const int idx = blockIdx.x * HOP_SP_THREADS + threadIdx.x;
+    int p = par_out, ieo = idx;
+    if (npar == 2)
+      {
+        p = (idx >= g.Vh) ? 1 : 0;
+        ieo = idx - (p ? (int)g.Vh : 0);
+      }
+    const bool active = (idx < npar * g.Vh);
     double part = 0.0;
     if (active)
       {
@@ -639,9 +644,14 @@ namespace tms
     extern __shared__ __align__(16) char spp_smem[];
     pdl_enter();
     if (stop && *stop) return;
-    const int p = (npar == 2) ? blockIdx.x & 1 : par_out; // both parities: alternating blocks, as in hop_kernel
-    const int ieo = ((npar == 2) ? blockIdx.x >> 1 : blockIdx.x) * SPP_THREADS + threadIdx.x;
-    const bool active = (ieo < g.Vh);
+    const int idx = blockIdx.x * SPP_THREADS + threadIdx.x;
+    int p = par_out, ieo = idx;
+    if (npar == 2)
+      {
+        p = (idx >= g.Vh) ? 1 : 0;
+        ieo = idx - (p ? (int)g.Vh : 0);
+      }
+    const bool active = (idx < npar * g.Vh);
     double part = 0.0;
     if (active)
       {

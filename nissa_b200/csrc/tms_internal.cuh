@@ -333,7 +333,7 @@ namespace tms_int
         auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
         static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         (void)attr;
-        launch_pdl(c, k, npar * div_up(c->g.Vh, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm, epi,
+        launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm, epi,
                    reducer(c), fin, stop);
         return;
       }
@@ -350,7 +350,7 @@ namespace tms_int
           {
             if (c->hop_cfg[P] == 5)
               {
-                launch_pdl(c, hop_sp_kernel<P, LF, Epi, Fin>, npar * div_up(c->g.Vh, HOP_SP_THREADS), HOP_SP_THREADS, 0, s, c->g,
+                launch_pdl(c, hop_sp_kernel<P, LF, Epi, Fin>, div_up(nsite, HOP_SP_THREADS), HOP_SP_THREADS, 0, s, c->g,
                            par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
                 return;
               }
@@ -364,7 +364,7 @@ namespace tms_int
                 auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
                 static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
                 (void)attr;
-                launch_pdl(c, k, npar * div_up(c->g.Vh, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm,
+                launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm,
                            epi, reducer(c), fin, stop);
                 return;
               }
@@ -411,15 +411,15 @@ namespace tms_int
         switch (c->hop_cfg[P])
           {
           case 1:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 1>, npar * div_up(c->g.Vh, HopCfg<P, 1>::NT), HopCfg<P, 1>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 1>, div_up(nsite, HopCfg<P, 1>::NT), HopCfg<P, 1>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
             break;
           case 2:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 2>, npar * div_up(c->g.Vh, HopCfg<P, 2>::NT), HopCfg<P, 2>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 2>, div_up(nsite, HopCfg<P, 2>::NT), HopCfg<P, 2>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
             break;
           default:
-            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 0>, npar * div_up(c->g.Vh, HopCfg<P, 0>::NT), HopCfg<P, 0>::NT, 0, s, c->g,
+            launch_pdl(c, hop_kernel<P, LF, Epi, Fin, 0>, div_up(nsite, HopCfg<P, 0>::NT), HopCfg<P, 0>::NT, 0, s, c->g,
                        par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
           }
       }
