@@ -316,7 +316,7 @@ uint64_t tms_launch_count(const tms_ctx *ctx);
 int64_t tms_hop_stage_timeouts(tms_ctx *ctx);
 /* Tuning knobs (no reference counterpart), used by the autotuner: "hop_cfg_double",
  * "hop_cfg_single", "hop_cfg_half" (hopping-kernel launch shape 0..2: one site per thread, 128 threads;
- * 128 threads with registers capped for 4 (FP64) / 8 resident blocks; 256 threads capped for 2 / 4;
+ * 128 threads with registers capped for 4 (FP64) / 6 resident blocks; 256 threads capped for 2 / 4;
  * single and half only, when T is a multiple of 4 (else shape 0 is used): 3 two sites (t, t+T/2) per
  * thread in packed FP32 arithmetic with the neighbours streamed through shared memory by cp.async,
  * 4 two sites per thread in packed FP32 arithmetic; for any T: 5 one site per thread with the two spin
@@ -346,7 +346,10 @@ int64_t tms_hop_stage_timeouts(tms_ctx *ctx);
  * about 15 % more iterations at 32^3x64 with the default reliable_delta_half, 3 % more and 3-5 % less time per
  * solve with reliable_delta_half 0.01),
  * "stream_priority" (the context's stream is recreated with this CUDA stream priority, an integer in the
- * device's range, lower first; contexts of small volumes sharing a GPU with large ones use it).  Results do not depend on the launch shapes. */
+ * device's range, lower first; contexts of small volumes sharing a GPU with large ones use it).  Results do not depend on the launch shapes.
+ * At its default value a shape also stands for the small-lattice kernels: launches of up to 6144
+ * (single: 9472) output sites spread a site's directions over a block, and the e/o twisted-mass CG
+ * of up to 9472 sites per parity runs up to 64 iterations in one cooperative launch. */
 tms_status tms_set_tuning(tms_ctx *ctx, const char *key, double value);
 /* The current value of a tuning knob (the keys of tms_set_tuning). */
 tms_status tms_get_tuning(tms_ctx *ctx, const char *key, double *value);

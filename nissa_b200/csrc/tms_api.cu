@@ -107,6 +107,7 @@ tms_status tms_create4(tms_ctx** out, int T, int LX, int LY, int LZ, double bc_t
       cudaMalloc(&ctx->st, sizeof(CgState)) != cudaSuccess ||
       cudaMalloc(&ctx->red_partial, sizeof(double) * ctx->red_cap) != cudaSuccess ||
       cudaMalloc(&ctx->red_counter, sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc(&ctx->grid_bar, sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&ctx->red_result, sizeof(double)) != cudaSuccess ||
       cudaMalloc(&ctx->tma_timeouts, sizeof(unsigned)) != cudaSuccess ||
       cudaHostAlloc(&ctx->st_h, sizeof(CgState), cudaHostAllocMapped) != cudaSuccess ||
@@ -179,6 +180,7 @@ tms_status tms_destroy(tms_ctx* ctx)
   fr(ctx->st);
   fr(ctx->red_partial);
   fr(ctx->red_counter);
+  fr(ctx->grid_bar);
   fr(ctx->tma_timeouts);
   fr(ctx->slab_ghost);
   fr(ctx->red_result);

@@ -1,6 +1,7 @@
 // C ABI of the e/o solvers: the CG of K(+mu)K(-mu) (FP64, and FP32 / FP16
 // inner with FP64 reliable updates) and the full solve of Eq. (8)-(11).
 #include "tms_solver.cuh"
+#include "tms_cg_small.cuh"
 
 using namespace tms_int;
 
@@ -10,6 +11,7 @@ namespace
   {
     static constexpr int slot0 = kSlotEo;
     static constexpr bool kHalfArith = true; // has the FP16-arithmetic hop
+    static constexpr bool kOneLaunch = true; // has the one-launch CG (tms_cg_small.cuh)
     static constexpr int nlo = 6;
     static int stride(tms_ctx* c) { return c->g.stride; }
     static int nsites(tms_ctx* c) { return (int)c->g.Vh; }
@@ -49,6 +51,60 @@ namespace
         n, view<PREC_F64>(b), view<PREC_F64>(s), view<PREC_F64>(r), reducer(ctx));
       CU(cudaGetLastError());
       *rr = read_result(ctx);
+      return TMS_OK;
+    }
+
+    // The one-launch CG: the default hop shape, and every 32-site block resident
+    // at once (two per SM: up to 9472 sites of a parity).  Whole solves, launches /
+    // one launch, at 864, 4096, 6400 and 9216 sites: FP64 2.13 / 2.10, 3.13 / 2.95,
+    // 4.05 / 3.24, 4.08 / 3.67 ms; FP32 2.22 / 1.84, 2.98 / 2.53, 3.03 / 2.69,
+    // 3.41 / 2.91; FP16 2.34 / 1.83, 3.23 / 2.45, 3.43 / 2.60, 3.47 / 2.79.
+    static constexpr int coherent(int P) { return P == PREC_F64 ? PREC_C64 : P == PREC_F32 ? PREC_C32 : PREC_C16; }
+    template <int P, int LF>
+    static auto one_kernel()
+    {
+      return cg_small_kernel<coherent(P), (P == PREC_F64) ? PREC_C64 : PREC_C32, LF>;
+    }
+    static constexpr int kOneIters = 64; // iterations of a launch: a bound on its length
+    template <int P, int LF>
+    static bool one_launch(tms_ctx* c)
+    {
+      const int blocks = div_up(c->g.Vh, HOP_DP_SITES);
+      if (c->hop_cfg[P] != HOP_CFG_DEFAULT[P]) return false;
+      int coop = 0, sms = 0, per = 0;
+      if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop ||
+          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, one_kernel<P, LF>(), HOP_DP_THREADS, 0) != cudaSuccess)
+        return false;
+      return blocks <= per * sms;
+    }
+    template <int P>
+    static SpinorT<P> past_l1(const Field& f)
+    {
+      SpinorT<P> s;
+      s.d = reinterpret_cast<decltype(s.d)>(f.d);
+      s.n = f.n;
+      s.stride = f.stride;
+      return s;
+    }
+    template <int P, int LF>
+    static tms_status launch_one(tms_ctx* ctx, const LinkT<LF>& U, const Field* v, const Field& x)
+    {
+      constexpr int PC = coherent(P), PXC = (P == PREC_F64) ? PREC_C64 : PREC_C32;
+      Lattice g = ctx->g;
+      SpinorT<PC> r = past_l1<PC>(v[1]), p = past_l1<PC>(v[2]), t1 = past_l1<PC>(v[3]), te = past_l1<PC>(v[4]);
+      SpinorT<PXC> xx = past_l1<PXC>(x);
+      LinkT<LF> u = U;
+      const OpParams* prm = ctx->prm;
+      CgState* st = ctx->st;
+      double* partial = ctx->red_partial;
+      unsigned* bar = ctx->grid_bar;
+      int iters = kOneIters;
+      void* args[] = {&g, &r, &p, &t1, &te, &xx, &u, &prm, &st, &partial, &bar, &iters};
+      ctx->launches += 2;
+      grid_bar_reset_kernel<<<1, 1, 0, ctx->stream>>>(bar);
+      CU(cudaLaunchCooperativeKernel((const void*)one_kernel<P, LF>(), dim3(div_up(g.Vh, HOP_DP_SITES)), dim3(HOP_DP_THREADS),
+                                     args, 0, ctx->stream));
       return TMS_OK;
     }
 

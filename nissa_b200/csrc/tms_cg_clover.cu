@@ -12,6 +12,7 @@ namespace
   {
     static constexpr int slot0 = kSlotClov;
     static constexpr bool kHalfArith = false;
+    static constexpr bool kOneLaunch = false;
     static constexpr bool kPaired = true;
     static Field& p2(tms_ctx* c) { return c->lo[5]; }
     static constexpr int nlo = 6;

@@ -10,6 +10,7 @@ namespace
   {
     static constexpr int slot0 = kSlotLx;
     static constexpr bool kHalfArith = false;
+    static constexpr bool kOneLaunch = false;
     static constexpr bool kPaired = false;
     static constexpr int nlo = 5;
     static int stride(tms_ctx* c) { return 2 * c->g.stride; }

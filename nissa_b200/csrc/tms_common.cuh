@@ -32,7 +32,8 @@
 
 namespace tms
 {
-  enum Prec { PREC_F64 = 0, PREC_F32 = 1, PREC_F16 = 2, PREC_A64 = 3 }; // A64: FP64 in the caller's layout (tms_hop_aos.cuh)
+  enum Prec { PREC_F64 = 0, PREC_F32 = 1, PREC_F16 = 2, PREC_A64 = 3, // A64: FP64 in the caller's layout (tms_hop_aos.cuh)
+              PREC_C64 = 4, PREC_C32 = 5, PREC_C16 = 6 };          // F64, F32, F16 read past L1 (tms_cg_small.cuh)
   enum LinkFmt { LINK_F64_18 = 0, LINK_F32_12 = 1, LINK_F32_18 = 2, LINK_I16_12 = 3, LINK_F64_12 = 4, LINK_H16_12 = 5 };
 
   // ------------------------------------------------------------- geometry

@@ -131,6 +131,47 @@ namespace tms
     reconstruct<D / 2, !(D & 1)>(acc, u0, u1);
   }
 
+  // direction d of a site (parity p, neighbour n): its products into the share
+  template <int P, int LF>
+  __device__ __forceinline__ void dp_direction(DpShare<typename SpinorT<P>::R>& sh, int d, int lane, int n, const SpinorT<P>& in,
+                                               const C<typename SpinorT<P>::R> L[9], typename SpinorT<P>::R ls)
+  {
+    using R = typename SpinorT<P>::R;
+    R ss;
+    C<R> v[12], a[3], b[3], u0[3], u1[3];
+    in.load_raw(n, v, ss);
+    const bool cross = dp_cross(d);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      {
+        a[c] = {cross ? v[9 + c].re : v[6 + c].re, cross ? v[9 + c].im : v[6 + c].im};
+        b[c] = {cross ? v[6 + c].re : v[9 + c].re, cross ? v[6 + c].im : v[9 + c].im};
+      }
+    dp_products<R>(d, v, v + 3, a, b, L, ss * ls, u0, u1);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      {
+        sh.u[d][c][lane] = u0[c];
+        sh.u[d][3 + c][lane] = u1[c];
+      }
+  }
+
+  template <typename R>
+  __device__ __forceinline__ void dp_sum(const DpShare<R>& sh, const Lattice& g, const Site& s, int lane, R anis,
+                                         C<R> acc[12])
+  {
+#pragma unroll
+    for (int c = 0; c < 12; c++) acc[c] = {R(0), R(0)};
+    dp_add<0>(sh, lane, (s.t == g.T - 1) ? R(g.bc_t) : R(1), acc);
+    dp_add<1>(sh, lane, (s.t == 0) ? R(g.bc_t) : R(1), acc);
+    dp_add<2>(sh, lane, anis, acc);
+    dp_add<3>(sh, lane, anis, acc);
+    dp_add<4>(sh, lane, anis, acc);
+    dp_add<5>(sh, lane, anis, acc);
+    dp_add<6>(sh, lane, anis, acc);
+    dp_add<7>(sh, lane, anis, acc);
+  }
+
   template <int P, int LF, class Epi, class Fin>
   __global__ void __launch_bounds__(HOP_DP_THREADS, 2)
     hop_dp_kernel(Lattice g, int par_out, int npar, SpinorT<P> in_e, SpinorT<P> in_o, LinkT<LF> U, const OpParams* prm,
@@ -146,44 +187,17 @@ namespace tms
     const Site s = eo_site(g, p, ieo);
     const int n = dp_neighbour(g, s, d) >> 1;
     C<R> L[9];
-    R ls, ss;
+    R ls;
     U.template load_scaled<false>((d & 1) ? 1 - p : p, d >> 1, (d & 1) ? n : ieo, L, ls);
     pdl_enter();
     if (stop && *stop) return; // the same for the whole grid: this kernel writes it after its last block's hop
-    {
-      C<R> v[12], a[3], b[3], u0[3], u1[3];
-      (p ? in_e : in_o).load_raw(n, v, ss);
-      const bool cross = dp_cross(d);
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        {
-          a[c] = {cross ? v[9 + c].re : v[6 + c].re, cross ? v[9 + c].im : v[6 + c].im};
-          b[c] = {cross ? v[6 + c].re : v[9 + c].re, cross ? v[6 + c].im : v[9 + c].im};
-        }
-      dp_products<R>(d, v, v + 3, a, b, L, ss * ls, u0, u1);
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        {
-          sh.u[d][c][lane] = u0[c];
-          sh.u[d][3 + c][lane] = u1[c];
-        }
-    }
+    dp_direction<P, LF>(sh, d, lane, n, p ? in_e : in_o, L, ls);
     __syncthreads();
     double part = 0.0;
     if (d == 0 && active)
       {
         C<R> acc[12];
-#pragma unroll
-        for (int c = 0; c < 12; c++) acc[c] = {R(0), R(0)};
-        const R anis = R(prm->anis);
-        dp_add<0>(sh, lane, (s.t == g.T - 1) ? R(g.bc_t) : R(1), acc);
-        dp_add<1>(sh, lane, (s.t == 0) ? R(g.bc_t) : R(1), acc);
-        dp_add<2>(sh, lane, anis, acc);
-        dp_add<3>(sh, lane, anis, acc);
-        dp_add<4>(sh, lane, anis, acc);
-        dp_add<5>(sh, lane, anis, acc);
-        dp_add<6>(sh, lane, anis, acc);
-        dp_add<7>(sh, lane, anis, acc);
+        dp_sum(sh, g, s, lane, R(prm->anis), acc);
         part = epi(p, ieo, acc);
       }
     if (Epi::kReduce) grid_reduce<HOP_DP_THREADS>(part, red, fin);

@@ -70,6 +70,7 @@ struct tms_ctx
   OpParams* prm = nullptr;       // [2]: operator params (slot 0 solver, slot 1 free use)
   CgState* st = nullptr;         // device solver state
   CgState* st_h = nullptr;       // pinned host mirror
+  unsigned* grid_bar = nullptr;  // barrier count of the one-launch CG
   double* red_partial = nullptr;
   unsigned* red_counter = nullptr;
   double* red_result = nullptr;
@@ -312,9 +313,11 @@ namespace tms_int
   // The shape of each precision unless tuned otherwise.  It stands for a rule:
   // launches of at most HOP_DP_SITES_MAX output sites run the direction-parallel
   // kernel instead.  Whole solves, shape / direction-parallel, at 4096, 4800 and
-  // 8400 sites: FP64 4.12 / 3.06, 3.59 / 2.95, 5.54 / 6.17 ms; FP32 4.45 / 2.99,
-  // 4.08 / 2.85, 5.09 / 4.66 (10368: 5.68 / 5.96); FP16 3.47 / 3.23, 3.14 / 2.85,
-  // 3.94 / 4.53.
+  // 16800 sites: FP64 4.12 / 3.06, 3.59 / 2.95, 5.54 / 6.17 ms; FP32 4.45 / 2.99,
+  // 4.08 / 2.85, 5.09 / 4.66 (20736: 5.68 / 5.96); FP16 3.47 / 3.23, 3.14 / 2.85,
+  // 3.94 / 4.53.  (The e/o solvers of these sizes run in one launch instead where
+  // they can, tms_cg_small.cuh: the rule is left to the full-lattice solvers, the
+  // FP64 steps around a solve, and other devices' residency.)
   constexpr int HOP_CFG_DEFAULT[3] = {0, 1, 6};
   constexpr int HOP_DP_SITES_MAX[3] = {6144, 9472, 6144};
 
@@ -447,12 +450,12 @@ namespace tms_int
   // caller's arrays directly; the others convert to planes and back around hops
   // on planes.  (A single hop, tms_hop_eo or tms_apply_tmQ, is direct at every
   // size: 32^3x64 hop 424 us, 440 with the conversions.)  Whole calls, direct /
-  // on planes: K^2 at 8400 sites 63.9 / 71.2 us, 20736 72.2 / 79.4, 36864
-  // 91.2 / 87.4, 331776 547 / 459; twisted-clover K^2 at 4096 45.7 / 67.5, 8400
+  // on planes: K^2 at 16800 sites 63.9 / 71.2 us, 20736 72.2 / 79.4, 36864
+  // 91.2 / 87.4, 331776 547 / 459; twisted-clover K^2 at 4096 45.7 / 67.5, 16800
   // 68.6 / 73.2, 20736 84.5 / 81.8.  The directions' products are spread over a
   // block, so nothing of a neighbour is reused through L1, which costs the more
   // the more sites there are to hide latencies.
-  constexpr int64_t AOS_KERN_SITES = 25000, AOS_Q2_SITES = 60000, AOS_CLOVER_SITES = 10000;
+  constexpr int64_t AOS_KERN_SITES = 25000, AOS_Q2_SITES = 60000, AOS_CLOVER_SITES = 18000;
 
   // one hop from `in` to epi.out, both in the caller's layout: e/o order of
   // parity par_out, or (FULL) lx order; the parameters travel with the launch

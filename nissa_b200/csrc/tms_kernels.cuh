@@ -523,7 +523,8 @@ namespace tms
     int dir;           // paired batched CG: which buffer holds the direction after a cut (set by the host)
   };
 
-  enum StopCode { STOP_RUN = 0, STOP_CONVERGED = 1, STOP_MAXITER = 2, STOP_RELIABLE = 3, STOP_BREAKDOWN = 4 };
+  enum StopCode { STOP_RUN = 0, STOP_CONVERGED = 1, STOP_MAXITER = 2, STOP_RELIABLE = 3, STOP_BREAKDOWN = 4,
+                  STOP_TIMEOUT = 6 }; // (5: an idle slot of a batch session)
 
   // alpha = rr / (p, A p)
   struct FinAlpha

@@ -61,6 +61,22 @@ namespace tms_int
     return TMS_OK;
   }
 
+  // One block of iterations: the policy's one-launch kernel where it applies
+  // (decided once a solve by one_launch), else the captured graph
+  template <class Op, int P, int LF>
+  bool one_launch(tms_ctx* ctx)
+  {
+    if constexpr (Op::kOneLaunch && LF != LINK_H16_12) return Op::template one_launch<P, LF>(ctx);
+    else return false;
+  }
+  template <class Op, int P, int LF>
+  tms_status run_block(tms_ctx* ctx, int slot, bool one, const LinkT<LF>& U, const Field* v, const Field& x)
+  {
+    if constexpr (Op::kOneLaunch && LF != LINK_H16_12)
+      if (one) return Op::template launch_one<P, LF>(ctx, U, v, x);
+    return launch_graph(ctx, slot);
+  }
+
   inline void fill_stats(tms_stats* stats, tms_status st, int iters, int reliable, double it_res, double true_res, float ms)
   {
     if (!stats) return;
@@ -105,13 +121,15 @@ namespace tms_int
     auto U = links64(ctx);
     Field v[5] = {Field{}, f[2], f[3], f[4], f[5]};
     const int slot = Op::slot0;
-    TRY(capture(ctx, slot, [&](cudaStream_t cs) {
-      Op::template record<PREC_F64, PREC_F64>(ctx, cs, U, v, f[1], ctx->graph_iters);
-    }));
+    const bool one = one_launch<Op, PREC_F64, LINK_F64_18>(ctx);
+    if (!one)
+      TRY(capture(ctx, slot, [&](cudaStream_t cs) {
+        Op::template record<PREC_F64, PREC_F64>(ctx, cs, U, v, f[1], ctx->graph_iters);
+      }));
     CU(cudaEventRecord(ctx->ev0, ctx->stream));
     while (S.stop == STOP_RUN)
       {
-        TRY(launch_graph(ctx, slot));
+        TRY(run_block<Op, PREC_F64>(ctx, slot, one, U, v, f[1]));
         TRY(pull_state(ctx));
       }
     CU(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -121,6 +139,7 @@ namespace tms_int
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     tms_status st = TMS_OK;
     if (S.stop == STOP_BREAKDOWN) st = fail(ctx, TMS_ERR_NAN, "nanned (iteration %d)", S.iter);
+    else if (S.stop == STOP_TIMEOUT) st = fail(ctx, TMS_ERR_TIMEOUT, "grid barrier (iteration %d)", S.iter);
     else if (S.stop == STOP_MAXITER) st = fail(ctx, TMS_ERR_NOT_CONVERGED, "exit without converging");
     fill_stats(stats, st, S.iter, 0, S.rr / b2, tr / b2, ms);
     return st;
@@ -189,18 +208,25 @@ namespace tms_int
         S.stop = STOP_RUN;
         TRY(push_state(ctx));
         Field v[5] = {Field{}, lo[1], lo[2], lo[3], lo[4]};
+        const bool one = one_launch<Op, P, LF>(ctx);
         // x updated every other iteration (e/o operator, even replay length)
-        const bool paired = Op::kPaired && ctx->graph_iters % 2 == 0;
-        TRY(capture(ctx, slot, [&](cudaStream_t cs) {
-          Op::template record<P, PX>(ctx, cs, U, v, xlo, ctx->graph_iters, paired);
-        }));
+        const bool paired = !one && Op::kPaired && ctx->graph_iters % 2 == 0;
+        if (!one)
+          TRY(capture(ctx, slot, [&](cudaStream_t cs) {
+            Op::template record<P, PX>(ctx, cs, U, v, xlo, ctx->graph_iters, paired);
+          }));
         CU(cudaEventRecord(ctx->ev0, ctx->stream));
         for (;;)
           {
             const int iter0 = S.iter;
-            TRY(launch_graph(ctx, slot));
+            TRY(run_block<Op, P>(ctx, slot, one, U, v, xlo));
             TRY(pull_state(ctx));
             if (S.stop == STOP_RUN) continue;
+            if (S.stop == STOP_TIMEOUT)
+              {
+                st = fail(ctx, TMS_ERR_TIMEOUT, "grid barrier (iteration %d)", S.iter);
+                break;
+              }
             if (S.stop == STOP_BREAKDOWN)
               {
                 st = fail(ctx, TMS_ERR_NAN, "nanned (iteration %d)", S.iter);

@@ -276,3 +276,34 @@ def test_columns_error_leaves_context_usable(cuda_device):
         sols, sts = lat.inv_tmD_cg_eoprec_columns(0.16, 0.01, [srcs[0], srcs[2]], 100000, 1e-20, precision="half")
         ref, _ = lat.inv_tmD_cg_eoprec(0.16, 0.01, srcs[2], 100000, 1e-20, precision="half")
         assert np.array_equal(sols[1], ref) and all(s["status"] == 0 for s in sts)
+
+
+@pytest.mark.parametrize("precision,other", [("double", 2), ("single", 0), ("half", 5)])
+@pytest.mark.parametrize("T,L", [(2, 4), (4, 6), (16, 8), (18, 10), (20, 10)])
+def test_one_launch_cg_equals_launches(cuda_device, T, L, precision, other):
+    """The CG in one cooperative launch (every 32-site block resident) against the launch-by-launch form, which a
+    non-default hop shape selects: 64, 432 (a ragged last block), 4096, 9000 (282 blocks, two per SM) and 10000
+    sites (too many blocks: launches on both sides); converged, cut by niter, and started from a guess."""
+    conf = wl.gauge_conf(T, L, 0.35, seed=T + L)
+    src = wl.random_spinor(T * L ** 3 // 2, 81)
+    got = []
+    with Lattice(T, L) as lat:
+        lat.upload_conf(conf)
+        for cfg in (None, other):
+            if cfg is not None:
+                lat.set_tuning("hop_cfg_" + precision, cfg)
+            sol, st = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 10000, 1e-22, precision=precision)
+            cut, sc = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 7, 1e-22, precision=precision,
+                                                           raise_on_error=False)
+            warm, sw = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 10000, 1e-22, guess=cut,
+                                                            precision=precision)
+            assert st["status"] == 0 and sw["status"] == 0 and sc["status"] == 1 and sc["iterations"] == 7
+            assert st["true_rel_res2"] < 1e-22 and sw["true_rel_res2"] < 1e-22
+            assert sw["iterations"] < st["iterations"]
+            got.append((sol, cut, warm, st["iterations"]))
+    (a, ca, wa, na), (b, cb, wb, nb) = got
+    # two solutions within 1e-11 of |b| in residue, cond(K K^+) below 1e3 here; FP32 and FP16 recurrences round
+    # differently, so their iteration counts may differ by a few
+    assert rel(a, b) < 1e-9 and rel(wa, wb) < 1e-9
+    assert rel(ca, cb) < (1e-12 if precision == "double" else 1e-2)
+    assert abs(na - nb) <= (1 if precision == "double" else 3 + nb // 8), (na, nb)
