@@ -316,7 +316,7 @@ uint64_t tms_launch_count(const tms_ctx *ctx);
 int64_t tms_hop_stage_timeouts(tms_ctx *ctx);
 /* Tuning knobs (no reference counterpart), used by the autotuner: "hop_cfg_double",
  * "hop_cfg_single", "hop_cfg_half" (hopping-kernel launch shape 0..2: one site per thread, 128 threads;
- * 128 threads with registers capped for 4 (FP64) / 6 resident blocks; 256 threads capped for 2 / 4;
+ * 128 threads with registers capped for 4 (FP64) / 8 resident blocks; 256 threads capped for 2 / 4;
  * single and half only, when T is a multiple of 4 (else shape 0 is used): 3 two sites (t, t+T/2) per
  * thread in packed FP32 arithmetic with the neighbours streamed through shared memory by cp.async,
  * 4 two sites per thread in packed FP32 arithmetic; for any T: 5 one site per thread with the two spin

@@ -931,15 +931,15 @@ namespace tms
   // par_out only, npar = 2 both parities (grid over 2*Vh).
   // Launch shapes the autotuner chooses from (per precision):
   //   CFG 0: 128 threads, no register cap
-  //   CFG 1: 128 threads, registers capped for 4 (FP64) / 6 (FP32, FP16) resident blocks per SM
-  //          (80 registers; capped for 8, at 64, the FP32 hops spill 88-120 bytes a thread:
-  //          24^3x48 FP32-inner solve 21.1 ms, 20.4 with 6; multi-shift 216 ms, 208)
+  //   CFG 1: 128 threads, registers capped for 4 (FP64) / 8 (FP32, FP16) resident blocks per SM
+  //          (64 registers, 88-120 bytes spilled; capped for 6, at 80, the multi-shift solve
+  //          at 24^3x48 takes 208 ms instead of 216, but the columns at 16^3x32 81.8 instead of 73.7)
   //   CFG 2: 256 threads, registers capped for 2 (FP64) / 4 (FP32, FP16) resident blocks per SM
   template <int P, int CFG>
   struct HopCfg
   {
     static constexpr int NT = (CFG == 2) ? 256 : 128;
-    static constexpr int MINB = (CFG == 0) ? 1 : (CFG == 1) ? (P == PREC_F64 ? 4 : 6) : (P == PREC_F64 ? 2 : 4);
+    static constexpr int MINB = (CFG == 0) ? 1 : (CFG == 1) ? (P == PREC_F64 ? 4 : 8) : (P == PREC_F64 ? 2 : 4);
   };
   constexpr int HOP_CFGS = 3;      // launch shapes of the one-site kernel
   constexpr int HOP_CFGS_ALL = 8;  // FP32 arithmetic: 3 the two-site packed kernel with the cp.async
