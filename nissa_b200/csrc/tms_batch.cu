@@ -159,8 +159,7 @@ namespace
           // one right-hand side per thread, gathers pipelined through shared memory
           constexpr int smem = SppFmt<P, LF>::template smem<MrhsPipe<P>::DIST>();
           auto k = hop_mrhs_kernel<P, LF, Epi, Fin, 1, true>;
-          static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-          (void)attr;
+          kernel_attr(c, k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
           k<<<w->grid, threads, smem, s>>>(c->g, par_out, nrhs, bview<P>(in), U, w->bp, epi, w->red, fin, st);
           return;
         }
@@ -400,8 +399,11 @@ namespace
       }
     w->nodes[slot] = ctx->launches - before;
     ctx->launches = before;
+    const cudaError_t launched = cudaGetLastError(); // a refused launch leaves its node out of the graph
     cudaError_t e = cudaStreamEndCapture(cs, &graph);
     cudaStreamDestroy(cs);
+    if (e == cudaSuccess && launched != cudaSuccess) cudaGraphDestroy(graph);
+    if (launched != cudaSuccess) e = launched;
     if (e != cudaSuccess) return fail(ctx, TMS_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     e = cudaGraphInstantiate(&w->graph[slot], graph, 0);
     cudaGraphDestroy(graph);

@@ -9,6 +9,7 @@
 #include "tms_hop_tma.cuh"
 #include "tms_hop_aos.cuh"
 #include "tms_clover.cuh"
+#include "tms_attr.cuh"
 
 #include <cmath>
 #include <cstdarg>
@@ -162,6 +163,8 @@ struct tms_ctx
   // kernels launched by this context (graph replays count their nodes)
   uint64_t launches = 0;
 
+  tms_int::KernelAttrs attrs; // of this context's device
+
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
   // pipelined host-buffer column solves: a copy stream, two source and two
@@ -291,6 +294,14 @@ namespace tms_int
   inline LinkT<LINK_F64_18> links64(tms_ctx* c) { return LinkT<LINK_F64_18>{c->U64, (int)c->g.Vh}; }
 
   // ------------------------------------------------------------ hop launch
+  // an attribute of a kernel on the context's device; a failure is left to the
+  // launch that needs it and to the check of the last error after it
+  template <class K>
+  void kernel_attr(tms_ctx* c, K* k, cudaFuncAttribute a, int v)
+  {
+    (void)c->attrs.once((const void*)k, (int)a, v, [&] { return cudaFuncSetAttribute(k, a, v); });
+  }
+
   // a launch with programmatic stream serialisation (when enabled): the kernel
   // may start while its predecessor drains; it waits in pdl_enter()
   template <typename... KArgs, typename... Args>
@@ -334,8 +345,7 @@ namespace tms_int
         constexpr int DIST = 2, MINB = 5;
         constexpr int smem = SppFmt<P, LF>::template smem<DIST>();
         auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
-        static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        (void)attr;
+        kernel_attr(c, k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm, epi,
                    reducer(c), fin, stop);
         return;
@@ -365,8 +375,7 @@ namespace tms_int
                 constexpr int MINB = (P == PREC_F16) ? 5 : 3;
                 constexpr int smem = SppFmt<P, LF>::template smem<DIST>();
                 auto k = hop_spp_kernel<P, LF, Epi, Fin, DIST, MINB>;
-                static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-                (void)attr;
+                kernel_attr(c, k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
                 launch_pdl(c, k, div_up(nsite, SPP_THREADS), SPP_THREADS, smem, s, c->g, par_out, npar, in_e, in_o, U, prm,
                            epi, reducer(c), fin, stop);
                 return;
@@ -381,12 +390,9 @@ namespace tms_int
                       const size_t smem = tma_smem_bytes<P, LF>(G.nc, G.ns);
                       auto k = hop_tma_kernel<P, LF, Epi, Fin>;
                       // the largest tile: at most HOP_TMA_THREADS sites and two halo rows of at most 64 sites
-                      static const cudaError_t a1 = cudaFuncSetAttribute(
-                        k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                        (int)tma_smem_bytes<P, LF>(HOP_TMA_THREADS + 128, HOP_TMA_THREADS));
-                      static const cudaError_t a2 = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-                      (void)a1;
-                      (void)a2;
+                      kernel_attr(c, k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)tma_smem_bytes<P, LF>(HOP_TMA_THREADS + 128, HOP_TMA_THREADS));
+                      kernel_attr(c, k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
                       launch_pdl(c, k, ntiles, HOP_TMA_THREADS, smem, s, c->g, G, par_out, npar, in_e, in_o, U, prm, epi,
                                  reducer(c), fin, stop);
                       return;
@@ -403,9 +409,7 @@ namespace tms_int
               else
                 {
                   constexpr int smem = PipeFmt<P, LF>::SMEM;
-                  static const cudaError_t attr = cudaFuncSetAttribute(
-                    hop_pipe_kernel<P, LF, Epi, Fin>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-                  (void)attr;
+                  kernel_attr(c, hop_pipe_kernel<P, LF, Epi, Fin>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
                   launch_pdl(c, hop_pipe_kernel<P, LF, Epi, Fin>, div_up(n2, PIPE_THREADS), PIPE_THREADS, smem, s, c->g,
                              par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);
                 }
@@ -463,8 +467,7 @@ namespace tms_int
   void launch_hop_aos(tms_ctx* c, int par_out, const double* in, const OpParams& prm, const Epi& epi)
   {
     auto k = hop_aos_dp_kernel<Epi, FULL>;
-    static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, AOS_DP_SMEM);
-    (void)attr;
+    kernel_attr(c, k, cudaFuncAttributeMaxDynamicSharedMemorySize, AOS_DP_SMEM);
     ++c->launches;
     launch_pdl(c, k, div_up(FULL ? c->g.V : c->g.Vh, HOP_DP_SITES), HOP_DP_THREADS, AOS_DP_SMEM, c->stream, c->g, par_out,
                reinterpret_cast<const double2*>(in), links64(c), prm, epi);

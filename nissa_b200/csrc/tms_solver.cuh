@@ -34,8 +34,11 @@ namespace tms_int
     rec(cs);
     ctx->graph_nodes[slot] = ctx->launches - before;
     ctx->launches = before;
+    const cudaError_t launched = cudaGetLastError(); // a refused launch leaves its node out of the graph
     cudaError_t e = cudaStreamEndCapture(cs, &graph);
     cudaStreamDestroy(cs);
+    if (e == cudaSuccess && launched != cudaSuccess) cudaGraphDestroy(graph);
+    if (launched != cudaSuccess) e = launched;
     if (e != cudaSuccess) return fail(ctx, TMS_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     e = cudaGraphInstantiate(&ctx->graph[slot], graph, 0);
     cudaGraphDestroy(graph);
