@@ -18,8 +18,21 @@ LIB = os.path.join(HERE, "libtmsolve.so")
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 
+# No --split-compile: it optimises a unit in parts, and the code of a kernel then depends on what else its
+# unit holds.  The batched FP64 hop, its source unchanged, came out such that 8 right-hand sides at
+# 24x12x10x14 took 83 or 52 ms, and 12 FP16 ones at 24^3x48 190 or 174 ms; FP32 solves at 24^3x48 20.8 or
+# 20.1 ms.  Without it every kernel has one form, the faster one of these, and the build is no slower
+# (130 instead of 155 s on 8 cores).  The exception is the FP16 twisted-mass CG, in a unit of its own:
+# its hops are better split (32^3x64 49.2 instead of 50.4 ms).
+SPLIT_UNITS = ("tms_cg_half.cu",)
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-              "-Xcompiler", "-fPIC", "-shared", "--expt-relaxed-constexpr", "--split-compile", "0"]
+              "-Xcompiler", "-fPIC", "-shared", "--expt-relaxed-constexpr"]
+
+
+def unit_flags(src: str) -> list:
+    """Compiler flags of one unit (to an object)."""
+    flags = [f for f in NVCC_FLAGS if f != "-shared"] + ["-I" + INCLUDE, "-I" + CSRC]
+    return flags + (["--split-compile", "0"] if os.path.basename(src) in SPLIT_UNITS else [])
 
 
 def sources():
@@ -54,8 +67,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         for src in sources():
             obj = os.path.join(d, os.path.basename(src) + ".o")
             objs.append(obj)
-            cmds.append([nvcc()] + [f for f in NVCC_FLAGS if f != "-shared"] + ["-I" + INCLUDE, "-I" + CSRC, "-c", src,
-                                                                               "-o", obj])
+            cmds.append([nvcc()] + unit_flags(src) + ["-c", src, "-o", obj])
         with concurrent.futures.ThreadPoolExecutor(max_workers=len(cmds)) as ex:
             for cmd, rc in zip(cmds, ex.map(lambda c: subprocess.call(c), cmds)):
                 if verbose:

@@ -301,6 +301,17 @@ namespace tms_int
   }
 
   template <class Op>
+  tms_status cg_half(tms_ctx* ctx, int niter, double residue, bool have_guess, tms_stats* stats)
+  {
+    // the e/o twisted-mass solver may run its hops in FP16 arithmetic (tuning "half_arith")
+    if constexpr (Op::kHalfArith)
+      if (ctx->su3 && ctx->half_arith)
+        return cg_mixed<Op, PREC_F16>(ctx, links16h(ctx), niter, residue, have_guess, stats);
+    return ctx->su3 ? cg_mixed<Op, PREC_F16>(ctx, links16r(ctx), niter, residue, have_guess, stats)
+                    : cg_mixed<Op, PREC_F16>(ctx, links32f(ctx), niter, residue, have_guess, stats);
+  }
+
+  template <class Op>
   tms_status cg_dispatch(tms_ctx* ctx, int precision, int niter, double residue, bool have_guess, tms_stats* stats)
   {
     if (precision == TMS_PREC_DOUBLE) return cg_double<Op>(ctx, niter, residue, have_guess, stats);
@@ -310,15 +321,7 @@ namespace tms_int
         return ctx->single_links16 ? cg_mixed<Op, PREC_F32>(ctx, links16r(ctx), niter, residue, have_guess, stats)
                                    : cg_mixed<Op, PREC_F32>(ctx, links32r(ctx), niter, residue, have_guess, stats);
       }
-    if (precision == TMS_PREC_MIXED_HALF)
-      {
-        // the e/o twisted-mass solver may run its hops in FP16 arithmetic (tuning "half_arith")
-        if constexpr (Op::kHalfArith)
-          if (ctx->su3 && ctx->half_arith)
-            return cg_mixed<Op, PREC_F16>(ctx, links16h(ctx), niter, residue, have_guess, stats);
-        return ctx->su3 ? cg_mixed<Op, PREC_F16>(ctx, links16r(ctx), niter, residue, have_guess, stats)
-                        : cg_mixed<Op, PREC_F16>(ctx, links32f(ctx), niter, residue, have_guess, stats);
-      }
+    if (precision == TMS_PREC_MIXED_HALF) return cg_half<Op>(ctx, niter, residue, have_guess, stats);
     return fail(ctx, TMS_ERR_BAD_ARG, "unknown precision %d", precision);
   }
 
