@@ -347,9 +347,10 @@ int64_t tms_hop_stage_timeouts(tms_ctx *ctx);
  * solve with reliable_delta_half 0.01),
  * "stream_priority" (the context's stream is recreated with this CUDA stream priority, an integer in the
  * device's range, lower first; contexts of small volumes sharing a GPU with large ones use it).  Results do not depend on the launch shapes.
- * At its default value a shape also stands for the small-lattice kernels: launches of up to 6144
- * (single: 9472) output sites spread a site's directions over a block, and the e/o twisted-mass CG
- * of up to 9472 sites per parity runs up to 64 iterations in one cooperative launch. */
+ * "small_lattice" (1, the default, or 0): the kernels for small lattices, whatever the shapes.  Launches of
+ * up to 6144 (single: 9472) output sites spread a site's directions over a block, the e/o twisted-mass CG of
+ * up to 9472 sites per parity runs up to 64 iterations in one cooperative launch, and small operators of
+ * several hops work on the caller's arrays.  With 0 the shapes hold at every size. */
 tms_status tms_set_tuning(tms_ctx *ctx, const char *key, double value);
 /* The current value of a tuning knob (the keys of tms_set_tuning). */
 tms_status tms_get_tuning(tms_ctx *ctx, const char *key, double *value);

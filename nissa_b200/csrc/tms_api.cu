@@ -320,7 +320,7 @@ static tms_status kern_common(tms_ctx* ctx, double kappa, int has_anis, double a
   OpBuffers b;
   TRY(op_begin(ctx, in, out, bytes, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.Vh > AOS_KERN_SITES)
+  if (ctx->g.Vh > AOS_KERN_SITES || !ctx->small_lattice)
     {
       Field &x = ctx->f64[6], &y = ctx->f64[7];
       TRY(alloc_field(ctx, x, PREC_F64));
@@ -364,7 +364,7 @@ static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double an
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
   OpBuffers b;
-  if (!square || ctx->g.V <= AOS_Q2_SITES)
+  if (!square || (ctx->g.V <= AOS_Q2_SITES && ctx->small_lattice))
     {
       Field& temp = ctx->lx64[6];
       if (square) TRY(alloc_field(ctx, temp, PREC_F64, 2 * ctx->g.stride));
@@ -438,6 +438,13 @@ tms_status tms_set_tuning(tms_ctx* ctx, const char* key, double value)
       if (v < 0 || v >= ncfg || v != value) return fail(ctx, TMS_ERR_BAD_ARG, "%s: 0..%d", key, ncfg - 1);
       if (ctx->hop_cfg[p] != v) drop_all();
       ctx->hop_cfg[p] = v;
+      return TMS_OK;
+    }
+  if (k == "small_lattice")
+    {
+      if (value != 0.0 && value != 1.0) return fail(ctx, TMS_ERR_BAD_ARG, "small_lattice: 0 or 1");
+      if (ctx->small_lattice != (int)value) drop_all();
+      ctx->small_lattice = (int)value;
       return TMS_OK;
     }
   if (k == "half_arith")
@@ -552,6 +559,7 @@ tms_status tms_get_tuning(tms_ctx* ctx, const char* key, double* value)
   else if (k == "hop_cfg_single") *value = ctx->hop_cfg[PREC_F32];
   else if (k == "hop_cfg_half") *value = ctx->hop_cfg[PREC_F16];
   else if (k == "tma_rows") *value = ctx->tma_rows;
+  else if (k == "small_lattice") *value = ctx->small_lattice;
   else if (k == "half_arith") *value = ctx->half_arith;
   else if (k == "graph_iters") *value = ctx->graph_iters;
   else if (k == "batch_graph_iters") *value = ctx->batch_iters;

@@ -390,7 +390,7 @@ static tms_status clov_kern_common(tms_ctx* ctx, double kappa, int has_anis, dou
   OpBuffers b;
   TRY(op_begin(ctx, in, out, bytes, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.Vh > AOS_CLOVER_SITES)
+  if (ctx->g.Vh > AOS_CLOVER_SITES || !ctx->small_lattice)
     {
       Field &x = ctx->f64[6], &y = ctx->f64[7];
       TRY(alloc_field(ctx, x, PREC_F64));
@@ -435,7 +435,7 @@ tms_status tms_apply_tmclovQ(tms_ctx* ctx, double kappa, int has_anis, double an
   OpBuffers b;
   TRY(op_begin(ctx, in, out, bytes, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.V <= AOS_CLOVER_SITES)
+  if (ctx->g.V <= AOS_CLOVER_SITES && ctx->small_lattice)
     {
       const ClovT<PREC_A64> cl{ctx->cl64, ctx->icl64, (int)ctx->g.Vh};
       launch_hop_aos<true>(ctx, 0, b.in, prm,

@@ -53,8 +53,7 @@ namespace tms_int
       return TMS_OK;
     }
 
-    // The one-launch CG: the default hop shape, and every 32-site block resident
-    // at once (two per SM: up to 9472 sites of a parity).  Whole solves, launches /
+    // The one-launch CG: where every 32-site block is resident at once (two per SM: up to 9472 sites of a parity).  Whole solves, launches /
     // one launch, at 864, 4096, 6400 and 9216 sites: FP64 2.13 / 2.10, 3.13 / 2.95,
     // 4.05 / 3.24, 4.08 / 3.67 ms; FP32 2.22 / 1.84, 2.98 / 2.53, 3.03 / 2.69,
     // 3.41 / 2.91; FP16 2.34 / 1.83, 3.23 / 2.45, 3.43 / 2.60, 3.47 / 2.79.
@@ -69,7 +68,7 @@ namespace tms_int
     static bool one_launch(tms_ctx* c)
     {
       const int blocks = div_up(c->g.Vh, HOP_DP_SITES);
-      if (c->hop_cfg[P] != HOP_CFG_DEFAULT[P]) return false;
+      if (!c->small_lattice) return false;
       int coop = 0, sms = 0, per = 0;
       if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop ||
           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||

@@ -144,7 +144,8 @@ struct tms_ctx
 
   // tuning (tms_set_tuning): hopping-kernel launch shape per precision, the
   // reliable-update trigger of the mixed solvers
-  int hop_cfg[3] = {0, 1, 6}; // HOP_CFG_DEFAULT
+  int hop_cfg[3] = {0, 1, 6};
+  int small_lattice = 1; // the kernels for small lattices where their size rules say so (0: never)
   int tma_rows = 0; // lattice rows per tile of the staged hop (launch shape 7): 0 the most that fit
   double delta_single = 1e-3, delta_half = 0.005;
   int single_links16 = 1; // FP32-spinor inner solver on 16-bit fixed-point links (1) or FP32 12-real links (0)
@@ -321,15 +322,13 @@ namespace tms_int
     cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
   }
 
-  // The shape of each precision unless tuned otherwise.  It stands for a rule:
-  // launches of at most HOP_DP_SITES_MAX output sites run the direction-parallel
-  // kernel instead.  Whole solves, shape / direction-parallel, at 4096, 4800 and
-  // 16800 sites: FP64 4.12 / 3.06, 3.59 / 2.95, 5.54 / 6.17 ms; FP32 4.45 / 2.99,
+  // Launches of at most this many output sites run the direction-parallel kernel
+  // whatever the shape (tuning "small_lattice" turns it off).  Whole solves, default
+  // shape / direction-parallel, at 4096, 4800 and 16800 sites: FP64 4.12 / 3.06, 3.59 / 2.95, 5.54 / 6.17 ms; FP32 4.45 / 2.99,
   // 4.08 / 2.85, 5.09 / 4.66 (20736: 5.68 / 5.96); FP16 3.47 / 3.23, 3.14 / 2.85,
   // 3.94 / 4.53.  (The e/o solvers of these sizes run in one launch instead where
   // they can, tms_cg_small.cuh: the rule is left to the full-lattice solvers, the
   // FP64 steps around a solve, and other devices' residency.)
-  constexpr int HOP_CFG_DEFAULT[3] = {0, 1, 6};
   constexpr int HOP_DP_SITES_MAX[3] = {6144, 9472, 6144};
 
   template <int P, int LF, class Epi, class Fin = NoFin>
@@ -353,7 +352,7 @@ namespace tms_int
     else
       {
         if constexpr (!HasClover<Epi>::value)
-          if (nsite <= HOP_DP_SITES_MAX[P] && c->hop_cfg[P] == HOP_CFG_DEFAULT[P])
+          if (nsite <= HOP_DP_SITES_MAX[P] && c->small_lattice)
             {
               launch_pdl(c, hop_dp_kernel<P, LF, Epi, Fin>, npar * div_up(c->g.Vh, HOP_DP_SITES), HOP_DP_THREADS, 0, s,
                          c->g, par_out, npar, in_e, in_o, U, prm, epi, reducer(c), fin, stop);

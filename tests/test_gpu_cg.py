@@ -222,6 +222,7 @@ def test_paired_x_updates_match_unpaired(cuda_device, precision):
     sols, its = [], []
     with Lattice(T, L) as lat:
         lat.upload_conf(conf)
+        lat.set_tuning("small_lattice", 0)  # in graph replays, where x updates are paired
         for gi in (8, 7, 2):
             lat.set_tuning("graph_iters", gi)
             sol, st = lat.inv_tmD_cg_eoprec(0.1610, 0.005, src, 100000, 1e-20, precision=precision)
@@ -278,20 +279,19 @@ def test_columns_error_leaves_context_usable(cuda_device):
         assert np.array_equal(sols[1], ref) and all(s["status"] == 0 for s in sts)
 
 
-@pytest.mark.parametrize("precision,other", [("double", 2), ("single", 0), ("half", 5)])
+@pytest.mark.parametrize("precision", ["double", "single", "half"])
 @pytest.mark.parametrize("T,L", [(2, 4), (4, 6), (16, 8), (18, 10), (20, 10)])
-def test_one_launch_cg_equals_launches(cuda_device, T, L, precision, other):
-    """The CG in one cooperative launch (every 32-site block resident) against the launch-by-launch form, which a
-    non-default hop shape selects: 64, 432 (a ragged last block), 4096, 9000 (282 blocks, two per SM) and 10000
+def test_one_launch_cg_equals_launches(cuda_device, T, L, precision):
+    """The CG in one cooperative launch (every 32-site block resident) against the launch-by-launch form in the
+    default hop shapes, which small_lattice 0 selects: 64, 432 (a ragged last block), 4096, 9000 (282 blocks, two per SM) and 10000
     sites (too many blocks: launches on both sides); converged, cut by niter, and started from a guess."""
     conf = wl.gauge_conf(T, L, 0.35, seed=T + L)
     src = wl.random_spinor(T * L ** 3 // 2, 81)
     got = []
     with Lattice(T, L) as lat:
         lat.upload_conf(conf)
-        for cfg in (None, other):
-            if cfg is not None:
-                lat.set_tuning("hop_cfg_" + precision, cfg)
+        for small in (1, 0):
+            lat.set_tuning("small_lattice", small)
             sol, st = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 10000, 1e-22, precision=precision)
             cut, sc = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 7, 1e-22, precision=precision,
                                                            raise_on_error=False)
@@ -307,3 +307,22 @@ def test_one_launch_cg_equals_launches(cuda_device, T, L, precision, other):
     assert rel(a, b) < 1e-9 and rel(wa, wb) < 1e-9
     assert rel(ca, cb) < (1e-12 if precision == "double" else 1e-2)
     assert abs(na - nb) <= (1 if precision == "double" else 3 + nb // 8), (na, nb)
+
+
+@pytest.mark.parametrize("precision,shape", [("double", 2), ("single", 0), ("half", 5)])
+def test_a_tuned_shape_keeps_the_one_launch_cg(cuda_device, precision, shape):
+    """A hop shape chosen for the launches of larger lattices leaves a 6400-site solve in one cooperative launch per
+    up to 64 iterations; small_lattice 0 gives the five launches of every iteration."""
+    V = 20 * 8 * 8 * 10
+    src = wl.random_spinor(V // 2, 91)
+    with Lattice(20, 0, LX=8, LY=8, LZ=10) as lat:
+        lat.upload_conf(wl.gauge_conf(V, 1, 0.35, seed=9))  # independent links: any V of them
+        counts = []
+        for shape_, small in ((None, 1), (shape, 1), (shape, 0)):
+            if shape_ is not None:
+                lat.set_tuning("hop_cfg_" + precision, shape_)
+            lat.set_tuning("small_lattice", small)
+            n0 = lat.launch_count
+            _, st = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 10000, 1e-18, precision=precision)
+            counts.append((lat.launch_count - n0) / st["iterations"])
+        assert counts[0] < 3 and counts[1] < 3 and counts[2] > 5, counts

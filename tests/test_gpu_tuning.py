@@ -38,6 +38,7 @@ def test_hop_shapes_agree(cuda_device, T, L, precision):
     with Lattice(T, L) as lat:
         lat.upload_conf(conf)
         ref, st0 = lat.inv_tmDkern_eoprec_square_eos_cg(KAPPA, MU, src, 100000, 1e-22)
+        lat.set_tuning("small_lattice", 0)  # the shapes themselves
         links = [0, 1] if precision == "single" else [0]
         for ls in links:
             lat.set_tuning("links_single", ls)
@@ -59,6 +60,7 @@ def test_tile_rows_agree(cuda_device, T, L, precision):
     with Lattice(T, L) as lat:
         lat.upload_conf(conf)
         ref, st0 = lat.inv_tmDkern_eoprec_square_eos_cg(KAPPA, MU, src, 100000, 1e-22)
+        lat.set_tuning("small_lattice", 0)
         lat.set_tuning("hop_cfg_" + precision, tune.TILED_SHAPE)
         rows = tune.tile_rows_choices(L, L)
         assert rows
@@ -103,6 +105,7 @@ def test_full_lattice_packed(cuda_device):
     with Lattice(T, L) as lat:
         lat.upload_conf(conf)
         ref, _ = lat.inv_tmQ2_cg(KAPPA, MU, src, 100000, 1e-22)
+        lat.set_tuning("small_lattice", 0)
         for prec in ("single", "half"):
             for v in (0, 3, 4, 5, 6, 7):
                 lat.set_tuning("hop_cfg_" + prec, v)
@@ -120,6 +123,10 @@ def test_shape_range_checked(cuda_device):
         lat.set_tuning("hop_cfg_half", 7)
         assert lat.get_tuning("hop_cfg_half") == 7 and lat.get_tuning("hop_cfg_single") == 1
         assert lat.get_tuning("tma_rows") == 0 and lat.get_tuning("reliable_delta_half") == 0.005
+        assert lat.get_tuning("small_lattice") == 1
+        for bad in (-1, 2, 0.5):
+            with pytest.raises(TmError):
+                lat.set_tuning("small_lattice", bad)
         with pytest.raises(TmError):
             lat.get_tuning("no_such_knob")
 

@@ -21,6 +21,9 @@ class FakeLattice:
     def set_tuning(self, k, v):
         self.knobs[k] = v
 
+    def get_tuning(self, k):
+        return self.knobs.get(k, 1 if k == "small_lattice" else 0)
+
     def bench_hop(self, precision, variant=0, nrep=10, flush=True):
         self.calls += 1
         shape = self.knobs.get("hop_cfg_" + precision, 0)
@@ -116,3 +119,35 @@ def test_record_capture_keeps_ncu_evidence(tmp_path):
         pass
     else:
         raise AssertionError("a capture without a tuned entry is refused")
+
+
+def test_shapes_are_timed_without_the_small_lattice_kernels(tmp_path):
+    cache = str(tmp_path / "t.json")
+    for before in (0, 1):
+        lat = FakeLattice()
+        lat.knobs["small_lattice"] = before
+        seen = []
+        bench = lat.bench_hop
+        lat.bench_hop = lambda *a, **k: (seen.append(lat.knobs["small_lattice"]), bench(*a, **k))[1]
+        assert "small_lattice" not in tune.autotune(lat, "half", device_name="dev", cache=cache, retune=True)["settings"]
+        assert seen and not any(seen) and lat.knobs["small_lattice"] == before
+
+    def broken(*a, **k):
+        raise RuntimeError
+    lat.bench_hop = broken
+    try:
+        tune.autotune(lat, "half", device_name="dev", cache=cache, retune=True)
+    except RuntimeError:
+        pass
+    assert lat.knobs["small_lattice"] == 1
+
+
+def test_entries_of_another_version_are_tuned_again(tmp_path):
+    cache = str(tmp_path / "t.json")
+    key = "dev|8x4x4x4|half|1"
+    for old in ({}, {"version": tune.VERSION - 1}):
+        json.dump({key: dict(old, settings={"hop_cfg_half": 5}, ms_per_iteration=1.0)}, open(cache, "w"))
+        lat = FakeLattice(best_shape=6)
+        r = tune.autotune(lat, "half", device_name="dev", cache=cache)
+        assert not r["cached"] and r["settings"] == {"hop_cfg_half": 6}
+        assert json.load(open(cache))[key]["version"] == tune.VERSION
