@@ -282,9 +282,7 @@ namespace tms
   }
 
   __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-  __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
   __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-  __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
   // diag_apply with the component a run-time value, contracted as the compiler
   // contracts it for a constant one, so that the results are the same bits
   template <typename R>
@@ -499,9 +497,12 @@ namespace tms
     __device__ __forceinline__ void comp(int p, int ieo, int c, C<R> acc, C<R> z) const
     {
       const C<R> xv = pick(x[0], x[1], p).load1(ieo, c);
-      const C<R> im = {-z.im * xv.im, z.im * xv.re}, h = cscale(acc, R(0.5)), k = cscale(xv, z.re);
-      acc = (c < 6) ? cadd(csub(k, h), im) : cadd(csub(h, k), im);
-      pick(out[0], out[1], p).store1(ieo, c, acc);
+      // contracted as the compiler contracts the site form: k - h keeps k's product, h - k rounds it (h is exact)
+      const bool up = c < 6;
+      const C<R> h = cscale(acc, R(0.5));
+      const C<R> s = {up ? fma_rn(xv.re, z.re, -h.re) : h.re - mul_rn(xv.re, z.re),
+                      up ? fma_rn(xv.im, z.re, -h.im) : h.im - mul_rn(xv.im, z.re)};
+      pick(out[0], out[1], p).store1(ieo, c, {fma_rn(-z.im, xv.im, s.re), fma_rn(z.im, xv.re, s.im)});
     }
   };
 

@@ -67,3 +67,23 @@ def test_operators_on_the_callers_layout(cuda_device, T, L, form):
         check(lambda i, o: lat.tmclovDkern_eoprec_square_eos(k, mu, i, anis=anis, out=o), x,
               geo.tmclov_kern2(ceo, k, Clo, inve, mu, x, anis=anis))
         check(lambda i, o: lat.apply_tmclovQ(k, mu, i, out=o), xl, geo.tmclovQ(cbc, k, Cl, mu, xl))
+
+
+def test_the_callers_layout_gives_the_bits_of_the_planes(cuda_device):
+    """The same operators from hops on planes (small_lattice 0): the components' forms of the epilogues round as the
+    sites' forms do, FMA for FMA.  (Q alone has no form on planes; Q^2 is made of it.)  The clover terms' sums of 6 to 12 products are
+    contracted differently: rounding, 1e-15."""
+    T, L = 10, 8
+    x, xl = wl.random_spinor(T * L ** 3 // 2, 73), wl.random_spinor(T * L ** 3, 74)
+    with Lattice(T, L) as lat:
+        lat.upload_conf(wl.gauge_conf(T, L, 0.35, seed=5))
+        lat.clover_term(1.3)
+        got = []
+        for small in (1, 0):
+            lat.set_tuning("small_lattice", small)
+            got.append([lat.tmDkern_eoprec_eos(0.14, 0.021, x, anis=1.15),
+                        lat.tmDkern_eoprec_square_eos(0.16, -0.5, x),
+                        lat.apply_tmQ2(0.14, 0.021, xl, anis=1.15), lat.apply_tmQ2(0.16, -0.5, xl),
+                        lat.tmclovDkern_eoprec_square_eos(0.13, 0.02, x, anis=1.15), lat.apply_tmclovQ(0.13, 0.02, xl)])
+        for k, (a, b) in enumerate(zip(*got)):
+            assert np.array_equal(a, b) if k < 4 else rel(a, b) < 1e-15, k
