@@ -350,7 +350,10 @@ int64_t tms_hop_stage_timeouts(tms_ctx *ctx);
  * "small_lattice" (1, the default, or 0): the kernels for small lattices, whatever the shapes.  Launches of
  * up to 6144 (single: 9472) output sites spread a site's directions over a block, the e/o twisted-mass CG of
  * up to 9472 sites per parity runs up to 64 iterations in one cooperative launch, and small operators of
- * several hops work on the caller's arrays.  With 0 the shapes hold at every size. */
+ * several hops work on the caller's arrays.  With 0 the shapes hold at every size.
+ * "grid_barrier_polls" (1 to 2^24, default 2^20, about a second): after as many polls a block of that launch
+ * gives up its wait for the others (which another stream's kernels may keep off the GPU); all then leave, and
+ * the solve goes on in launches from the FP64 solution it has. */
 tms_status tms_set_tuning(tms_ctx *ctx, const char *key, double value);
 /* The current value of a tuning knob (the keys of tms_set_tuning). */
 tms_status tms_get_tuning(tms_ctx *ctx, const char *key, double *value);

@@ -447,6 +447,13 @@ tms_status tms_set_tuning(tms_ctx* ctx, const char* key, double value)
       ctx->small_lattice = (int)value;
       return TMS_OK;
     }
+  if (k == "grid_barrier_polls")
+    {
+      const int v = (int)value;
+      if (v < 1 || v > (1 << 24) || v != value) return fail(ctx, TMS_ERR_BAD_ARG, "grid_barrier_polls: 1..2^24");
+      ctx->grid_polls = v;
+      return TMS_OK;
+    }
   if (k == "half_arith")
     {
       if (value != 0.0 && value != 1.0) return fail(ctx, TMS_ERR_BAD_ARG, "half_arith: 0 (FP32 arithmetic) or 1");
@@ -560,6 +567,7 @@ tms_status tms_get_tuning(tms_ctx* ctx, const char* key, double* value)
   else if (k == "hop_cfg_half") *value = ctx->hop_cfg[PREC_F16];
   else if (k == "tma_rows") *value = ctx->tma_rows;
   else if (k == "small_lattice") *value = ctx->small_lattice;
+  else if (k == "grid_barrier_polls") *value = ctx->grid_polls;
   else if (k == "half_arith") *value = ctx->half_arith;
   else if (k == "graph_iters") *value = ctx->graph_iters;
   else if (k == "batch_graph_iters") *value = ctx->batch_iters;

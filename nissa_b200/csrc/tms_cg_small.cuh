@@ -108,12 +108,13 @@ namespace tms
 
   // ------------------------------------------------------- grid barrier
   // All blocks of a cooperative launch arrive before any leaves.  The wait is
-  // bounded (about a second of polls): false if it gave up.
-  constexpr int GRID_BAR_POLLS = 1 << 20;
+  // bounded: false if it gave up.
+  constexpr int GRID_BAR_POLLS = 1 << 20; // about a second
   struct GridBarrier
   {
     unsigned* count; // 0 at launch
     unsigned target;
+    int limit; // polls
     __device__ __forceinline__ bool sync()
     {
       __syncthreads();
@@ -125,7 +126,7 @@ namespace tms
           unsigned v;
           int polls = 0;
           do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-          while (v < target && ++polls < GRID_BAR_POLLS);
+          while (v < target && ++polls < limit);
           ok = v >= target;
         }
       return __syncthreads_and(ok);
@@ -182,7 +183,8 @@ namespace tms
   template <int P, int PX, int LF>
   __global__ void __launch_bounds__(HOP_DP_THREADS, 2)
     cg_small_kernel(Lattice g, SpinorT<P> r, SpinorT<P> p, SpinorT<P> t1, SpinorT<P> te, SpinorT<PX> x, LinkT<LF> U,
-                    const OpParams* __restrict__ prm_g, CgState* st_g, double* partial, unsigned* bar_count, int iters)
+                    const OpParams* __restrict__ prm_g, CgState* st_g, double* partial, unsigned* bar_count, int polls,
+                    int iters)
   {
     using R = typename SpinorT<P>::R;
     __shared__ DpShare<R> sh;
@@ -199,7 +201,7 @@ namespace tms
     const int ieo = active ? blockIdx.x * HOP_DP_SITES + lane : (int)g.Vh - 1;
     const Site s0 = eo_site(g, 0, ieo), s1 = eo_site(g, 1, ieo);
     const int n0 = dp_neighbour(g, s0, d) >> 1, n1 = dp_neighbour(g, s1, d) >> 1;
-    GridBarrier bar{bar_count, 0u};
+    GridBarrier bar{bar_count, 0u, polls};
     __syncthreads();
     const R anis = R(prm.anis);
     bool alive = true;
@@ -234,6 +236,8 @@ namespace tms
           }
         if (!(alive = bar.sync())) break;
       }
+    // (a block that gave up stays away from the next barrier, so all give up there, or there is none: then
+    // the others have finished the launch's work, and so had it, and either outcome is right)
     if (threadIdx.x == 0)
       {
         if (!alive) st_g->stop = STOP_TIMEOUT;

@@ -2,7 +2,6 @@
 // (inv_tmDkern_eoprec_square_eos_cg).
 #pragma once
 #include "tms_solver.cuh"
-#include "tms_cg_small.cuh"
 
 namespace tms_int
 {
@@ -73,7 +72,10 @@ namespace tms_int
       if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop ||
           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, one_kernel<P, LF>(), HOP_DP_THREADS, 0) != cudaSuccess)
-        return false;
+        {
+          cudaGetLastError(); // the launches do without
+          return false;
+        }
       return blocks <= per * sms;
     }
     template <int P>
@@ -86,7 +88,8 @@ namespace tms_int
       return s;
     }
     template <int P, int LF>
-    static tms_status launch_one(tms_ctx* ctx, const LinkT<LF>& U, const Field* v, const Field& x)
+    // false if the device refuses the launch (fewer SMs for this process than the device has)
+    static bool launch_one(tms_ctx* ctx, const LinkT<LF>& U, const Field* v, const Field& x)
     {
       constexpr int PC = coherent(P), PXC = (P == PREC_F64) ? PREC_C64 : PREC_C32;
       Lattice g = ctx->g;
@@ -97,13 +100,15 @@ namespace tms_int
       CgState* st = ctx->st;
       double* partial = ctx->red_partial;
       unsigned* bar = ctx->grid_bar;
-      int iters = kOneIters;
-      void* args[] = {&g, &r, &p, &t1, &te, &xx, &u, &prm, &st, &partial, &bar, &iters};
+      int polls = ctx->grid_polls, iters = kOneIters;
+      void* args[] = {&g, &r, &p, &t1, &te, &xx, &u, &prm, &st, &partial, &bar, &polls, &iters};
       ctx->launches += 2;
       grid_bar_reset_kernel<<<1, 1, 0, ctx->stream>>>(bar);
-      CU(cudaLaunchCooperativeKernel((const void*)one_kernel<P, LF>(), dim3(div_up(g.Vh, HOP_DP_SITES)), dim3(HOP_DP_THREADS),
-                                     args, 0, ctx->stream));
-      return TMS_OK;
+      if (cudaLaunchCooperativeKernel((const void*)one_kernel<P, LF>(), dim3(div_up(g.Vh, HOP_DP_SITES)),
+                                      dim3(HOP_DP_THREADS), args, 0, ctx->stream) == cudaSuccess)
+        return true;
+      cudaGetLastError();
+      return false;
     }
 
     // the paired x update (record with paired = true) keeps the second direction here

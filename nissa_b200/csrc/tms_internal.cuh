@@ -8,6 +8,7 @@
 #include "tms_hop_sp.cuh"
 #include "tms_hop_tma.cuh"
 #include "tms_hop_aos.cuh"
+#include "tms_cg_small.cuh"
 #include "tms_clover.cuh"
 #include "tms_attr.cuh"
 
@@ -72,6 +73,7 @@ struct tms_ctx
   CgState* st = nullptr;         // device solver state
   CgState* st_h = nullptr;       // pinned host mirror
   unsigned* grid_bar = nullptr;  // barrier count of the one-launch CG
+  int grid_polls = GRID_BAR_POLLS; // after which its barrier gives up
   double* red_partial = nullptr;
   unsigned* red_counter = nullptr;
   double* red_result = nullptr;

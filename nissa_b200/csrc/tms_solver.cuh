@@ -64,19 +64,26 @@ namespace tms_int
     return TMS_OK;
   }
 
-  // One block of iterations: the policy's one-launch kernel where it applies
-  // (decided once a solve by one_launch), else the captured graph
+  // One block of iterations: the policy's one-launch kernel while it applies
+  // (`one`: decided at a solve's start by one_launch, and given up if the launch
+  // is refused or its barrier gives up), else the graph that prepare() captures
   template <class Op, int P, int LF>
   bool one_launch(tms_ctx* ctx)
   {
     if constexpr (Op::kOneLaunch && LF != LINK_H16_12) return Op::template one_launch<P, LF>(ctx);
     else return false;
   }
-  template <class Op, int P, int LF>
-  tms_status run_block(tms_ctx* ctx, int slot, bool one, const LinkT<LF>& U, const Field* v, const Field& x)
+  template <class Op, int P, int LF, class Prepare>
+  tms_status run_block(tms_ctx* ctx, int slot, bool& one, const Prepare& prepare, const LinkT<LF>& U, const Field* v,
+                       const Field& x)
   {
     if constexpr (Op::kOneLaunch && LF != LINK_H16_12)
-      if (one) return Op::template launch_one<P, LF>(ctx, U, v, x);
+      if (one)
+        {
+          if (Op::template launch_one<P, LF>(ctx, U, v, x)) return TMS_OK;
+          one = false;
+        }
+    TRY(prepare());
     return launch_graph(ctx, slot);
   }
 
@@ -124,16 +131,26 @@ namespace tms_int
     auto U = links64(ctx);
     Field v[5] = {Field{}, f[2], f[3], f[4], f[5]};
     const int slot = Op::slot0;
-    const bool one = one_launch<Op, PREC_F64, LINK_F64_18>(ctx);
-    if (!one)
-      TRY(capture(ctx, slot, [&](cudaStream_t cs) {
+    bool one = one_launch<Op, PREC_F64, LINK_F64_18>(ctx);
+    auto prepare = [&]() -> tms_status {
+      return capture(ctx, slot, [&](cudaStream_t cs) {
         Op::template record<PREC_F64, PREC_F64>(ctx, cs, U, v, f[1], ctx->graph_iters);
-      }));
+      });
+    };
+    if (!one) TRY(prepare());
     CU(cudaEventRecord(ctx->ev0, ctx->stream));
     while (S.stop == STOP_RUN)
       {
-        TRY(run_block<Op, PREC_F64>(ctx, slot, one, U, v, f[1]));
+        TRY(run_block<Op, PREC_F64>(ctx, slot, one, prepare, U, v, f[1]));
         TRY(pull_state(ctx));
+        if (S.stop != STOP_TIMEOUT) continue;
+        // the blocks left at different steps: on with the launches, from x as it is
+        one = false;
+        TRY(Op::true_residual(ctx, f[0], f[1], f[2], &rr));
+        CU(cudaMemcpyAsync(f[3].d, f[2].d, f[2].bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        S.rr = rr;
+        S.stop = (rr < S.target) ? STOP_CONVERGED : (S.iter >= niter) ? STOP_MAXITER : STOP_RUN;
+        TRY(push_state(ctx));
       }
     CU(cudaEventRecord(ctx->ev1, ctx->stream));
     double tr;
@@ -142,7 +159,6 @@ namespace tms_int
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     tms_status st = TMS_OK;
     if (S.stop == STOP_BREAKDOWN) st = fail(ctx, TMS_ERR_NAN, "nanned (iteration %d)", S.iter);
-    else if (S.stop == STOP_TIMEOUT) st = fail(ctx, TMS_ERR_TIMEOUT, "grid barrier (iteration %d)", S.iter);
     else if (S.stop == STOP_MAXITER) st = fail(ctx, TMS_ERR_NOT_CONVERGED, "exit without converging");
     fill_stats(stats, st, S.iter, 0, S.rr / b2, tr / b2, ms);
     return st;
@@ -211,24 +227,44 @@ namespace tms_int
         S.stop = STOP_RUN;
         TRY(push_state(ctx));
         Field v[5] = {Field{}, lo[1], lo[2], lo[3], lo[4]};
-        const bool one = one_launch<Op, P, LF>(ctx);
-        // x updated every other iteration (e/o operator, even replay length)
-        const bool paired = !one && Op::kPaired && ctx->graph_iters % 2 == 0;
-        if (!one)
-          TRY(capture(ctx, slot, [&](cudaStream_t cs) {
-            Op::template record<P, PX>(ctx, cs, U, v, xlo, ctx->graph_iters, paired);
-          }));
+        bool one = one_launch<Op, P, LF>(ctx);
+        // replays update x every other iteration (e/o operator, even replay length)
+        const bool pair = Op::kPaired && ctx->graph_iters % 2 == 0;
+        auto prepare = [&]() -> tms_status {
+          return capture(ctx, slot, [&](cudaStream_t cs) {
+            Op::template record<P, PX>(ctx, cs, U, v, xlo, ctx->graph_iters, pair);
+          });
+        };
+        if (!one) TRY(prepare());
         CU(cudaEventRecord(ctx->ev0, ctx->stream));
         for (;;)
           {
             const int iter0 = S.iter;
-            TRY(run_block<Op, P>(ctx, slot, one, U, v, xlo));
+            TRY(run_block<Op, P>(ctx, slot, one, prepare, U, v, xlo));
+            const bool paired = pair && !one;
             TRY(pull_state(ctx));
             if (S.stop == STOP_RUN) continue;
             if (S.stop == STOP_TIMEOUT)
               {
-                st = fail(ctx, TMS_ERR_TIMEOUT, "grid barrier (iteration %d)", S.iter);
-                break;
+                // the blocks left at different steps: on with the launches, from the
+                // FP64 solution of the last reliable update
+                one = false;
+                CU(cudaMemsetAsync(xlo.d, 0, xlo.bytes, ctx->stream));
+                TRY(Op::true_residual(ctx, f[0], f[1], f[2], &rr, true));
+                last_rt = rr;
+                if (rr < target) break;
+                if (S.iter >= niter)
+                  {
+                    st = fail(ctx, TMS_ERR_NOT_CONVERGED, "exit without converging");
+                    break;
+                  }
+                convert<P, PREC_F64>(ctx, f[2], lo[1], 1.0, n);
+                convert<P, PREC_F64>(ctx, f[2], lo[2], 1.0, n);
+                S.rr = rr;
+                S.rel_trigger = delta * delta * rr;
+                S.stop = STOP_RUN;
+                TRY(push_state(ctx));
+                continue;
               }
             if (S.stop == STOP_BREAKDOWN)
               {

@@ -326,3 +326,33 @@ def test_a_tuned_shape_keeps_the_one_launch_cg(cuda_device, precision, shape):
             _, st = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 10000, 1e-18, precision=precision)
             counts.append((lat.launch_count - n0) / st["iterations"])
         assert counts[0] < 3 and counts[1] < 3 and counts[2] > 5, counts
+
+
+@pytest.mark.parametrize("precision", ["double", "single", "half"])
+def test_barrier_that_gives_up_falls_back_to_launches(cuda_device, precision):
+    """With one poll allowed, blocks of the one-launch CG that do not arrive last give up, and all leave: the solve
+    goes on in launches and reaches its target, from zero and from a guess; the context's next solve, with the usual
+    limit, runs in one launch again."""
+    T, L = 16, 8
+    src = wl.random_spinor(T * L ** 3 // 2, 95)
+    args = (0.16, 0.01, src, 10000, 1e-22)
+    with Lattice(T, L) as lat:
+        lat.upload_conf(wl.gauge_conf(T, L, 0.35, seed=96))
+        ref, st0 = lat.inv_tmDkern_eoprec_square_eos_cg(*args, precision=precision)
+        default = lat.get_tuning("grid_barrier_polls")
+        lat.set_tuning("grid_barrier_polls", 1)
+        cut, sc = lat.inv_tmDkern_eoprec_square_eos_cg(0.16, 0.01, src, 7, 1e-22, precision=precision,
+                                                       raise_on_error=False)
+        assert sc["status"] == 1 and sc["iterations"] <= 7 + 64
+        for guess in (None, cut):
+            n0 = lat.launch_count
+            sol, st = lat.inv_tmDkern_eoprec_square_eos_cg(*args, guess=guess, precision=precision)
+            assert st["status"] == 0 and st["true_rel_res2"] < 1e-22 and rel(sol, ref) < 1e-9
+            assert (lat.launch_count - n0) / st["iterations"] > 5  # launches
+        lat.set_tuning("grid_barrier_polls", default)
+        n0 = lat.launch_count
+        sol, st = lat.inv_tmDkern_eoprec_square_eos_cg(*args, precision=precision)
+        assert (lat.launch_count - n0) / st["iterations"] < 3 and np.array_equal(sol, ref)
+        for bad in (0, 0.5, 1 << 25):
+            with pytest.raises(TmError):
+                lat.set_tuning("grid_barrier_polls", bad)
