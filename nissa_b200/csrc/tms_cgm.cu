@@ -90,33 +90,67 @@ namespace
     return w;
   }
 
-  // the residuals of a window besides the running one, as many as memory has room
-  // for: a window of `want` iterations, or of a divisor of it
-  tms_status ensure_window(tms_ctx* ctx, int prec, size_t fbytes, int want)
+  // The residuals of a window besides the running one.  They lie in full-lattice
+  // FP64 fields that are idle while the multi-shift iteration runs (what is in
+  // them is written anew after it): FP32 finds room for eight, FP64 for three.
+  // An FP64 window of more takes the rest from ctx->cgm_r, or is shortened to a
+  // divisor of `want` where memory is short.
+  struct CgmStore
   {
-    if (ctx->cgm_window && ctx->cgm_window_prec == prec && ctx->cgm_window_want == want) return TMS_OK;
-    TRY(drop_graph(ctx, 6));
-    TRY(drop_graph(ctx, 7));
+    std::vector<void*> r;
+    int window = 1;
+  };
+  constexpr size_t CGM_KEEP = (size_t)64 << 20; // ctx->cgm_r outlives the call up to this size
+
+  void drop_window(tms_ctx* ctx)
+  {
     if (ctx->cgm_r) cudaFree(ctx->cgm_r);
     ctx->cgm_r = nullptr;
-    ctx->cgm_window = 0;
-    // what the rest of the call may still allocate (the e/o solver's FP64 and inner
-    // fields, the staging buffer) stays free
+    ctx->cgm_r_bytes = 0;
+  }
+
+  tms_status find_window(tms_ctx* ctx, int prec, size_t fbytes, int want, CgmStore& st)
+  {
+    const bool hi = prec == PREC_F64;
+    std::vector<Field*> idle;
+    if (hi) idle = {&ctx->lx64[1], &ctx->lx64[5], &ctx->lx64[6]};
+    else idle = {&ctx->lx64[1], &ctx->lx64[2], &ctx->lx64[3], &ctx->lx64[4]};
+    // sites of the padding stay zero in every layout that a field is read in
+    if (ctx->g.stride != ctx->g.Vh)
+      for (Field* f : idle) CU(cudaMemsetAsync(f->d, 0, f->bytes, ctx->stream));
+    for (Field* f : idle)
+      for (size_t o = 0; o + fbytes <= f->bytes; o += fbytes) st.r.push_back((unsigned char*)f->d + o);
+    const int have = (int)st.r.size();
+    // what the rest of the call may still allocate stays free
     const size_t reserve = (size_t)32 * 192 * ctx->g.stride;
     int w = want;
     for (; w > 1; w--)
       {
         if (want % w) continue;
+        const size_t more = w - 1 > have ? fbytes * (w - 1 - have) : 0;
+        if (more <= ctx->cgm_r_bytes) break;
+        drop_window(ctx);
         size_t avail = 0, total = 0;
         CU(cudaMemGetInfo(&avail, &total));
-        if (avail < fbytes * (w - 1) + reserve) continue;
-        if (cudaMalloc(&ctx->cgm_r, fbytes * (w - 1)) == cudaSuccess) break;
+        if (avail < more + reserve) continue;
+        if (cudaMalloc(&ctx->cgm_r, more) == cudaSuccess)
+          {
+            ctx->cgm_r_bytes = more;
+            CU(cudaMemsetAsync(ctx->cgm_r, 0, more, ctx->stream));
+            break;
+          }
         ctx->cgm_r = nullptr;
         cudaGetLastError(); // out of memory: a shorter window
       }
-    ctx->cgm_window = w;
-    ctx->cgm_window_prec = prec;
-    ctx->cgm_window_want = want;
+    for (size_t o = 0; o + fbytes <= ctx->cgm_r_bytes; o += fbytes) st.r.push_back((unsigned char*)ctx->cgm_r + o);
+    st.window = w;
+    // a graph holds the addresses it was captured with
+    if (hi && (ctx->cgm_graph_window != w || ctx->cgm_graph_r != ctx->cgm_r))
+      {
+        TRY(drop_graph(ctx, 6));
+        ctx->cgm_graph_window = w;
+        ctx->cgm_graph_r = ctx->cgm_r;
+      }
     return TMS_OK;
   }
 
@@ -184,12 +218,13 @@ namespace
     const Field& r = hi ? ctx->lx64[2] : ctx->lxlo[1];
     const Field& p = hi ? ctx->lx64[3] : ctx->lxlo[2];
     const Field& t = hi ? ctx->lx64[4] : ctx->lxlo[3];
-    TRY(ensure_window(ctx, P, fbytes, cgm_window(ctx->graph_iters)));
+    CgmStore store;
+    TRY(find_window(ctx, P, fbytes, cgm_window(ctx->graph_iters), store));
     // the window's residuals: iteration j of a window writes R(j), reading its predecessor's
-    const int W = ctx->cgm_window;
+    const int W = store.window;
     auto R = [&](int j) {
       Field f = r;
-      if (j < W - 1) f.d = (unsigned char*)ctx->cgm_r + fbytes * j;
+      if (j < W - 1) f.d = store.r[j];
       return f;
     };
     // solution / direction views of shift k
@@ -257,6 +292,10 @@ namespace
     CU(cudaEventSynchronize(ctx->ev1));
     cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);
     *iters = S.iter;
+    if (ctx->cgm_r_bytes > CGM_KEEP) drop_window(ctx);
+    // the fields that held FP32 residuals are FP64 fields again
+    if (!hi && stride != 2 * ctx->g.Vh)
+      for (int i = 1; i <= 4; i++) CU(cudaMemsetAsync(ctx->lx64[i].d, 0, ctx->lx64[i].bytes, ctx->stream));
     if (S.stop == STOP_BREAKDOWN) return fail(ctx, TMS_ERR_NAN, "nanned (cgm iteration %d)", S.iter);
     if (S.stop == STOP_MAXITER) return fail(ctx, TMS_ERR_NOT_CONVERGED, "exit without converging");
     return TMS_OK;

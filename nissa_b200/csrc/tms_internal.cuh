@@ -120,8 +120,10 @@ struct tms_ctx
   void* cgm_x = nullptr;
   void* cgm_ps = nullptr;
   int cgm_prec = -1, cgm_nshift = 0;
-  void* cgm_r = nullptr; // residuals of a window of iterations besides the running one
-  int cgm_window = 0, cgm_window_prec = -1, cgm_window_want = 0;
+  void* cgm_r = nullptr; // residuals of an FP64 window of iterations that the idle fields have no room for
+  size_t cgm_r_bytes = 0;
+  int cgm_graph_window = 0;           // what the FP64 graph was captured with
+  const void* cgm_graph_r = nullptr;
 
   // lx spinor buffers on the device for the propagator entry points (tms_prop.cu)
   double* lxbuf[2] = {nullptr, nullptr};

@@ -99,3 +99,49 @@ def test_cgm_window_lengths(cuda_device, graph_iters, precision, niter):
             cond = (0.5 / 0.16 + 4) ** 2 / masses[k] ** 2
             tol = 1e-12 if precision == "double" else 0.2 * np.sqrt(res[k]) * min(cond, 1e3)
             assert rel(got[1][0][k], got[0][0][k]) < tol, k
+
+
+@pytest.mark.parametrize("precision", ["single", "half", "double"])
+def test_a_window_keeps_no_memory(cuda_device, precision):
+    """After a call a window of eight iterations holds what one of a single iteration does: the residuals lie in
+    fields that are idle meanwhile, and what FP64 needs beyond them is given back (64 MiB at most are kept)."""
+    import torch
+    T, L = 24, 16  # FP64: 18.9 MB a field, seven besides the running one
+    src = torch.from_numpy(wl.random_spinor(T * L ** 3, 47)).to("cuda:0")
+    conf = wl.gauge_conf(T, L, 0.35, seed=48, device="cuda")
+    used = []
+    for n in (8, 1):
+        with Lattice(T, L) as lat:
+            lat.upload_conf(conf)
+            lat.set_tuning("graph_iters", n)
+            out = [torch.empty_like(src) for _ in range(2)]
+            torch.cuda.synchronize()
+            free0 = torch.cuda.mem_get_info()[0]
+            lat.inv_tmQ2_cgm(0.15, [0.1, 0.5], src, 100000, [1e-16, 1e-16], precision=precision, out=out)
+            used.append(free0 - torch.cuda.mem_get_info()[0])
+    slack = 16 << 20  # the graphs' own memory
+    assert used[0] <= used[1] + slack, used
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_window_on_a_padded_lattice(cuda_device, precision):
+    """216 sites a parity in planes of 256: fields used before in the caller's layout (Q^2) or for FP32 residuals
+    leave nothing in the padding that a later reduction or solve could see."""
+    T, L = 2, 6
+    src = wl.random_spinor(T * L ** 3, 49)
+    masses, res = [0.05, 0.4], [1e-20, 1e-18]
+    with Lattice(T, L) as lat:
+        lat.upload_conf(wl.gauge_conf(T, L, 0.35, seed=50))
+        lat.apply_tmQ2(0.16, 0.1, src)
+        got = []
+        for n in (11, 8, 8):
+            lat.set_tuning("graph_iters", n)
+            got.append(lat.inv_tmQ2_cgm(0.16, masses, src, 100000, res, precision=precision))
+            sol, st = lat.inv_tmQ2_cg(0.16, 0.05, src, 100000, 1e-20)
+            assert st["true_rel_res2"] < 1e-20
+            for k, m in enumerate(masses):
+                r = lat.apply_tmQ2(0.16, m, got[-1][0][k]) - src
+                assert np.vdot(r, r) / np.vdot(src, src) < 1.01 * res[k]
+        for k in range(2):
+            assert np.array_equal(got[1][0][k], got[2][0][k])
+            assert rel(got[1][0][k], got[0][0][k]) < (1e-12 if precision == "double" else 1e-6)
