@@ -275,7 +275,7 @@ tms_status tms_hop_eo(tms_ctx* ctx, int par_out, const double* in, double* out, 
   if (par_out != 0 && par_out != 1) return fail(ctx, TMS_ERR_BAD_ARG, "parity must be 0 or 1");
   const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
   OpBuffers b;
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, OP_GATHER, b));
   const OpParams prm{1.0, 0.0, has_anis ? anis : 1.0};
   launch_hop_aos<false>(ctx, par_out, b.in, prm, EpiPlain<PREC_A64>{{view_aos(b.out), view_aos(b.out)}});
   return op_end(ctx, b, out, bytes);
@@ -288,7 +288,7 @@ static tms_status diag_common(tms_ctx* ctx, double kappa, double mu, const doubl
   TRY(check_params(ctx, kappa, mu));
   const size_t bytes = (size_t)ctx->g.Vh * 24 * sizeof(double);
   OpBuffers b;
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, OP_ELEMENTWISE, b));
   const int64_t n = ctx->g.Vh * 12;
   ++ctx->launches;
   diag_aos_kernel<<<div_up(n, 256), 256, 0, ctx->stream>>>(n, reinterpret_cast<const double2*>(b.in),
@@ -317,10 +317,11 @@ static tms_status kern_common(tms_ctx* ctx, double kappa, int has_anis, double a
   Field &te = ctx->f64[5], &t1 = ctx->f64[4];
   TRY(alloc_field(ctx, te, PREC_F64));
   if (square) TRY(alloc_field(ctx, t1, PREC_F64));
+  const bool planes = ctx->g.Vh > AOS_KERN_SITES || !ctx->small_lattice;
   OpBuffers b;
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, planes ? OP_PLANES : OP_GATHER, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.Vh > AOS_KERN_SITES || !ctx->small_lattice)
+  if (planes)
     {
       Field &x = ctx->f64[6], &y = ctx->f64[7];
       TRY(alloc_field(ctx, x, PREC_F64));
@@ -368,7 +369,7 @@ static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double an
     {
       Field& temp = ctx->lx64[6];
       if (square) TRY(alloc_field(ctx, temp, PREC_F64, 2 * ctx->g.stride));
-      TRY(op_begin(ctx, in, out, bytes, b));
+      TRY(op_begin(ctx, in, out, bytes, OP_GATHER, b));
       auto q = [&](const double* x, double* y, double sgn) {
         launch_hop_aos<true>(ctx, 0, x, prm,
                              EpiTmQ<PREC_A64, false>{{view_aos(y), view_aos(y)}, {view_aos(x), view_aos(x)}, nullptr, sgn});
@@ -379,7 +380,7 @@ static tms_status tmQ_common(tms_ctx* ctx, double kappa, int has_anis, double an
     }
   Field* f = ctx->f64;
   for (int i = 2; i <= 7; i++) TRY(alloc_field(ctx, f[i], PREC_F64));
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, OP_PLANES, b));
   TRY(put_params(ctx, prm));
   launch_lx_split(ctx, b.in, view<PREC_F64>(f[6]), view<PREC_F64>(f[7]));
   auto q = [&](int x, int y, double sgn) {

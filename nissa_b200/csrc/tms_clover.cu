@@ -387,10 +387,11 @@ static tms_status clov_kern_common(tms_ctx* ctx, double kappa, int has_anis, dou
   Field &te = ctx->f64[5], &t1 = ctx->f64[4];
   TRY(alloc_field(ctx, te, PREC_F64));
   if (square) TRY(alloc_field(ctx, t1, PREC_F64));
+  const bool planes = ctx->g.Vh > AOS_CLOVER_SITES || !ctx->small_lattice;
   OpBuffers b;
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, planes ? OP_PLANES : OP_GATHER, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.Vh > AOS_CLOVER_SITES || !ctx->small_lattice)
+  if (planes)
     {
       Field &x = ctx->f64[6], &y = ctx->f64[7];
       TRY(alloc_field(ctx, x, PREC_F64));
@@ -432,10 +433,11 @@ tms_status tms_apply_tmclovQ(tms_ctx* ctx, double kappa, int has_anis, double an
   TRY(check_clover(ctx));
   TRY(check_params(ctx, kappa, mu));
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
+  const bool planes = ctx->g.V > AOS_CLOVER_SITES || !ctx->small_lattice;
   OpBuffers b;
-  TRY(op_begin(ctx, in, out, bytes, b));
+  TRY(op_begin(ctx, in, out, bytes, planes ? OP_PLANES : OP_GATHER, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};
-  if (ctx->g.V <= AOS_CLOVER_SITES && ctx->small_lattice)
+  if (!planes)
     {
       const ClovT<PREC_A64> cl{ctx->cl64, ctx->icl64, (int)ctx->g.Vh};
       launch_hop_aos<true>(ctx, 0, b.in, prm,

@@ -509,23 +509,30 @@ namespace tms_int
   }
 
   // The buffers of one operator call: the caller's own where the kernels can
-  // work on them, else (host pointers, pointers off a 16-byte boundary, an input
-  // that overlaps the output) copies in the staging buffer.
+  // work on them, else copies in the staging buffer.
+  //   OP_GATHER       hops read the input while they write the output, in 16-byte
+  //                   words: no pointer off such a boundary, no overlap
+  //   OP_ELEMENTWISE  16-byte words; the output may be the input, not overlap it
+  //   OP_PLANES       the input is read, in any 8-byte words, before the output is written
+  enum OpUse { OP_GATHER, OP_ELEMENTWISE, OP_PLANES };
   struct OpBuffers
   {
     const double* in = nullptr;
     double* out = nullptr;
   };
-  inline tms_status op_begin(tms_ctx* ctx, const double* in, double* out, size_t bytes, OpBuffers& b)
+  inline tms_status op_begin(tms_ctx* ctx, const double* in, double* out, size_t bytes, OpUse use, OpBuffers& b)
   {
     const bool host = ctx->ptr_mode == TMS_PTR_HOST;
     if (!host && (!in || !out)) return fail(ctx, TMS_ERR_BAD_ARG, "null spinor");
     const uintptr_t i = (uintptr_t)in, o = (uintptr_t)out;
-    const bool copy_in = host || i % 16 || (i < o + bytes && o < i + bytes);
-    const bool copy_out = host || o % 16;
-    if (copy_in || copy_out) TRY(ensure_stage(ctx, 2 * bytes));
+    const bool overlap = i < o + bytes && o < i + bytes && !(use == OP_ELEMENTWISE && i == o);
+    const bool copy_in = host || (use != OP_PLANES && (i % 16 || overlap));
+    const bool copy_out = host || (use != OP_PLANES && o % 16);
+    // both copies in one place where the kernels may work in place
+    const bool two = copy_in && copy_out && use == OP_GATHER;
+    if (copy_in || copy_out) TRY(ensure_stage(ctx, two ? 2 * bytes : bytes));
     b.in = in;
-    b.out = copy_out ? ctx->stage + bytes / sizeof(double) : out;
+    b.out = copy_out ? ctx->stage + (two ? bytes / sizeof(double) : 0) : out;
     if (copy_in)
       {
         CU(cudaMemcpyAsync(ctx->stage, in, bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream));
