@@ -67,10 +67,10 @@ namespace tms
     return s;
   }
 
-  // lx index of the forward / backward neighbour in direction mu (0=t,1=x,2=y,3=z)
+  // e/o index of the forward / backward neighbour in direction mu (0=t,1=x,2=y,3=z)
   // and whether the hop crosses the time boundary
   template <int MU>
-  __device__ __forceinline__ int nbr_up_lx(const Lattice& g, const Site& s, bool& wrap_t)
+  __device__ __forceinline__ int nbr_up(const Lattice& g, const Site& s, bool& wrap_t)
   {
     int lx;
     wrap_t = false;
@@ -83,11 +83,11 @@ namespace tms
         wrap_t = (s.t == g.T - 1);
         lx = wrap_t ? s.lx - (g.T - 1) * st : s.lx + st;
       }
-    return lx;
+    return lx >> 1;
   }
 
   template <int MU>
-  __device__ __forceinline__ int nbr_dw_lx(const Lattice& g, const Site& s, bool& wrap_t)
+  __device__ __forceinline__ int nbr_dw(const Lattice& g, const Site& s, bool& wrap_t)
   {
     int lx;
     wrap_t = false;
@@ -100,20 +100,7 @@ namespace tms
         wrap_t = (s.t == 0);
         lx = wrap_t ? s.lx + (g.T - 1) * st : s.lx - st;
       }
-    return lx;
-  }
-
-  // their e/o indices
-  template <int MU>
-  __device__ __forceinline__ int nbr_up(const Lattice& g, const Site& s, bool& wrap_t)
-  {
-    return nbr_up_lx<MU>(g, s, wrap_t) >> 1;
-  }
-
-  template <int MU>
-  __device__ __forceinline__ int nbr_dw(const Lattice& g, const Site& s, bool& wrap_t)
-  {
-    return nbr_dw_lx<MU>(g, s, wrap_t) >> 1;
+    return lx >> 1;
   }
 
   // ---------------------------------------- programmatic dependent launch

@@ -10,11 +10,11 @@
 // memory and each lane reads its own record back at a pitch of 208 bytes, free
 // of bank conflicts; the output leaves as whole lines.
 // Whole calls, before (conversions around a hop on planes) / after: 8^3x16 hop
-// 49.8 / 32.7 us, 24^3x48 215 / 155 us, 32^3x64 561 / 424 us; 24^3x48 Q 450 /
-// 290 us.  (One warp for the eight directions of 32 sites, three directions
-// ahead, took 404 us a launch at 32^3x64 too, with eight warps per SM and the
-// copies' address exchange and the reads back queueing on the shared-memory pipe.; three
-// blocks per SM instead of two took 474 us, their shared memory being L1's.)
+// 46 / 20.8 us, 32^3x64 563 / 425 us; 24^3x48 Q 453 / 281 us.  (One warp for the
+// eight directions of 32 sites, three directions ahead, took 404 us a launch at
+// 32^3x64 too, with eight warps per SM: the copies' address exchange and the
+// reads back queue on the shared-memory pipe.  Three blocks per SM instead of
+// two took 474 us, their shared memory being L1's.)
 #pragma once
 
 #include <type_traits>
