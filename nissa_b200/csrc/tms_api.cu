@@ -33,7 +33,7 @@ namespace
                                                                                      view<P>(in), view<P>(in));
     void* scratch = nullptr;
     const size_t sbytes = size_t(512) << 20;
-    if (flush) CU(cudaMalloc(&scratch, sbytes));
+    if (flush) CU(dev_alloc(ctx, &scratch, sbytes));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -217,7 +217,7 @@ tms_status tms_geometry_tables(tms_ctx* ctx, int32_t* parity, int32_t* eo_of_lx,
   CU(cudaSetDevice(ctx->device));
   const int64_t V = ctx->g.V;
   int* d = nullptr;
-  CU(cudaMalloc(&d, sizeof(int) * V * 11));
+  CU(dev_alloc(ctx, &d, sizeof(int) * V * 11));
   ++ctx->launches;
   geometry_tables_kernel<<<div_up(V, 256), 256, 0, ctx->stream>>>(ctx->g, d, d + V, d + 2 * V, d + 3 * V, d + 7 * V);
   cudaError_t e = cudaGetLastError();
@@ -237,11 +237,11 @@ tms_status tms_conf_upload(tms_ctx* ctx, const double* conf, int layout, int fla
   CU(cudaSetDevice(ctx->device));
   const int64_t V = ctx->g.V, Vh = ctx->g.Vh;
   const size_t bytes = (size_t)V * 72 * sizeof(double);
-  if (!ctx->U64) CU(cudaMalloc(&ctx->U64, (size_t)V * 36 * sizeof(double2)));
-  if (!ctx->U32r) CU(cudaMalloc(&ctx->U32r, (size_t)V * 12 * sizeof(float4)));
-  if (!ctx->U32f) CU(cudaMalloc(&ctx->U32f, (size_t)V * 36 * sizeof(float2)));
-  if (!ctx->U16r) CU(cudaMalloc(&ctx->U16r, LinkT<LINK_I16_12>::bytes(ctx->g.Vh)));
-  if (!ctx->U16h) CU(cudaMalloc(&ctx->U16h, LinkT<LINK_H16_12>::bytes(ctx->g.Vh)));
+  if (!ctx->U64) CU(dev_alloc(ctx, &ctx->U64, (size_t)V * 36 * sizeof(double2)));
+  if (!ctx->U32r) CU(dev_alloc(ctx, &ctx->U32r, (size_t)V * 12 * sizeof(float4)));
+  if (!ctx->U32f) CU(dev_alloc(ctx, &ctx->U32f, (size_t)V * 36 * sizeof(float2)));
+  if (!ctx->U16r) CU(dev_alloc(ctx, &ctx->U16r, LinkT<LINK_I16_12>::bytes(ctx->g.Vh)));
+  if (!ctx->U16h) CU(dev_alloc(ctx, &ctx->U16h, LinkT<LINK_H16_12>::bytes(ctx->g.Vh)));
   const double* src = conf;
   if (ctx->ptr_mode == TMS_PTR_HOST)
     {

@@ -103,11 +103,11 @@ namespace
     f.stride = ctx->g.stride;
     f.nrhs = nrhs;
     f.bytes = planes_bytes(prec) * (size_t)f.stride * nrhs;
-    CU(cudaMalloc(&f.d, f.bytes));
+    CU(dev_alloc(ctx, &f.d, f.bytes));
     CU(cudaMemsetAsync(f.d, 0, f.bytes, ctx->stream));
     if (prec == PREC_F16)
       {
-        CU(cudaMalloc(&f.n, sizeof(float) * (size_t)f.stride * nrhs));
+        CU(dev_alloc(ctx, &f.n, sizeof(float) * (size_t)f.stride * nrhs));
         CU(cudaMemsetAsync(f.n, 0, sizeof(float) * (size_t)f.stride * nrhs, ctx->stream));
       }
     return TMS_OK;
@@ -124,13 +124,13 @@ namespace
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         w->grid = std::max(1, div_up(ctx->g.Vh, 32 * MRHS_WARPS)); // one 32-site chunk per warp
-        CU(cudaMalloc(&w->st, sizeof(CgState) * MRHS_MAX));
-        CU(cudaMalloc(&w->mask, sizeof(CgState) * MRHS_MAX));
-        CU(cudaMalloc(&w->bp, sizeof(BatchParams)));
+        CU(dev_alloc(ctx, &w->st, sizeof(CgState) * MRHS_MAX));
+        CU(dev_alloc(ctx, &w->mask, sizeof(CgState) * MRHS_MAX));
+        CU(dev_alloc(ctx, &w->bp, sizeof(BatchParams)));
         // rows long enough for the hop kernels' grid and the BLAS grid (blas_grid <= 592)
-        CU(cudaMalloc(&w->red.partial, sizeof(double) * MRHS_MAX * (size_t)std::max(w->grid, 592)));
-        CU(cudaMalloc(&w->red.counter, sizeof(unsigned) * MRHS_MAX));
-        CU(cudaMalloc(&w->red.result, sizeof(double) * MRHS_MAX));
+        CU(dev_alloc(ctx, &w->red.partial, sizeof(double) * MRHS_MAX * (size_t)std::max(w->grid, 592)));
+        CU(dev_alloc(ctx, &w->red.counter, sizeof(unsigned) * MRHS_MAX));
+        CU(dev_alloc(ctx, &w->red.result, sizeof(double) * MRHS_MAX));
         CU(cudaMemset(w->red.counter, 0, sizeof(unsigned) * MRHS_MAX));
         CU(cudaMallocHost(&w->st_h, sizeof(CgState) * MRHS_MAX));
         CU(cudaMallocHost(&w->mask_h, sizeof(CgState) * MRHS_MAX));
@@ -222,7 +222,7 @@ namespace
     CU(cudaMemcpyAsync(w->bp, w->bp_h, sizeof(BatchParams), cudaMemcpyHostToDevice, ctx->stream));
     void* scratch = nullptr;
     const size_t sbytes = size_t(512) << 20;
-    if (flush) CU(cudaMalloc(&scratch, sbytes));
+    if (flush) CU(dev_alloc(ctx, &scratch, sbytes));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);

@@ -135,7 +135,7 @@ namespace
         b = nullptr;
       }
     ctx->colbuf_bytes = 0;
-    for (double*& b : ctx->colbuf) CU(cudaMalloc(&b, bytes));
+    for (double*& b : ctx->colbuf) CU(dev_alloc(ctx, &b, bytes));
     ctx->colbuf_bytes = bytes;
     return TMS_OK;
   }

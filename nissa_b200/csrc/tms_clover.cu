@@ -310,10 +310,10 @@ tms_status tms_clover_term(tms_ctx* ctx, double cSW)
   TRY(check_conf(ctx));
   if (!std::isfinite(cSW)) return fail(ctx, TMS_ERR_BAD_ARG, "invalid cSW %g", cSW);
   const size_t Vh = ctx->g.Vh;
-  if (!ctx->cl64) CU(cudaMalloc(&ctx->cl64, 72 * Vh * sizeof(double2)));
-  if (!ctx->cl32) CU(cudaMalloc(&ctx->cl32, 72 * Vh * sizeof(float2)));
-  if (!ctx->icl64) CU(cudaMalloc(&ctx->icl64, 72 * Vh * sizeof(double2)));
-  if (!ctx->icl32) CU(cudaMalloc(&ctx->icl32, 72 * Vh * sizeof(float2)));
+  if (!ctx->cl64) CU(dev_alloc(ctx, &ctx->cl64, 72 * Vh * sizeof(double2)));
+  if (!ctx->cl32) CU(dev_alloc(ctx, &ctx->cl32, 72 * Vh * sizeof(float2)));
+  if (!ctx->icl64) CU(dev_alloc(ctx, &ctx->icl64, 72 * Vh * sizeof(double2)));
+  if (!ctx->icl32) CU(dev_alloc(ctx, &ctx->icl32, 72 * Vh * sizeof(float2)));
   // chromo_operator_include_cSW: Cl *= chromo_operator_factor(cSW + 1e-16) / chromo_operator_factor(-4)
   const double factor = (-(cSW + 1e-16) / 4) / (-(-4.0) / 4);
   const long long V = ctx->g.V;

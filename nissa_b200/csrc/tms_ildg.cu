@@ -339,7 +339,7 @@ tms_status tms_conf_plaquette(tms_ctx* ctx, int with_bc, double* plaquette)
   const Lattice& g = ctx->g;
   const int nb = (int)((g.V + PLAQ_THREADS - 1) / PLAQ_THREADS);
   double* buf = nullptr;
-  CU(cudaMalloc(&buf, sizeof(double) * (2 * (size_t)nb + 2)));
+  CU(dev_alloc(ctx, &buf, sizeof(double) * (2 * (size_t)nb + 2)));
   struct Freer
   {
     double* p;

@@ -211,6 +211,28 @@ namespace tms_int
     }                                                                                                            \
   while (0)
 
+  // frees the FP64 multi-shift window's residuals (tms_cgm.cu); between calls nothing uses them
+  inline void drop_window(tms_ctx* ctx)
+  {
+    if (ctx->cgm_r) cudaFree(ctx->cgm_r);
+    ctx->cgm_r = nullptr;
+    ctx->cgm_r_bytes = 0;
+  }
+
+  // device memory that stays with the context; a window that a multi-shift call kept gives way
+  template <class T>
+  cudaError_t dev_alloc(tms_ctx* ctx, T** p, size_t bytes)
+  {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->cgm_r)
+      {
+        cudaGetLastError();
+        drop_window(ctx);
+        e = cudaMalloc(p, bytes);
+      }
+    return e;
+  }
+
   inline tms_status alloc_field(tms_ctx* ctx, Field& f, int prec, int stride = 0)
   {
     if (stride == 0) stride = ctx->g.stride;
@@ -226,11 +248,11 @@ namespace tms_int
     f.stride = stride;
     const size_t per = (prec == PREC_F64) ? 192 : (prec == PREC_F32) ? 96 : 48;
     f.bytes = per * (size_t)f.stride;
-    CU(cudaMalloc(&f.d, f.bytes));
+    CU(dev_alloc(ctx, &f.d, f.bytes));
     CU(cudaMemsetAsync(f.d, 0, f.bytes, ctx->stream));
     if (prec == PREC_F16)
       {
-        CU(cudaMalloc(&f.n, sizeof(float) * (size_t)f.stride));
+        CU(dev_alloc(ctx, &f.n, sizeof(float) * (size_t)f.stride));
         CU(cudaMemsetAsync(f.n, 0, sizeof(float) * (size_t)f.stride, ctx->stream));
       }
     return TMS_OK;
@@ -242,7 +264,7 @@ namespace tms_int
     if (ctx->stage) cudaFree(ctx->stage);
     ctx->stage = nullptr;
     ctx->stage_bytes = 0;
-    CU(cudaMalloc(&ctx->stage, bytes));
+    CU(dev_alloc(ctx, &ctx->stage, bytes));
     ctx->stage_bytes = bytes;
     return TMS_OK;
   }

@@ -41,7 +41,7 @@ namespace
 
   tms_status ensure_lxbuf(tms_ctx* ctx, int k)
   {
-    if (!ctx->lxbuf[k]) CU(cudaMalloc(&ctx->lxbuf[k], (size_t)ctx->g.V * 24 * sizeof(double)));
+    if (!ctx->lxbuf[k]) CU(dev_alloc(ctx, &ctx->lxbuf[k], (size_t)ctx->g.V * 24 * sizeof(double)));
     return TMS_OK;
   }
 

@@ -171,7 +171,7 @@ namespace
     const int face = face_sites(ctx->g);
     const size_t bytes = (size_t)face * 6 * sizeof(double2);
     if (!ctx->slab_ghost)
-      CU(cudaMalloc(&ctx->slab_ghost, 2 * bytes));
+      CU(dev_alloc(ctx, &ctx->slab_ghost, 2 * bytes));
     double2* g0 = reinterpret_cast<double2*>(ctx->slab_ghost);
     const cudaMemcpyKind k = (ctx->ptr_mode == TMS_PTR_HOST) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     CU(cudaMemcpyAsync(g0, fwd, bytes, k, ctx->stream));
@@ -230,7 +230,7 @@ tms_status tms_slab_pack(tms_ctx* ctx, int par_in, const double* in, double* fac
   const int face = face_sites(ctx->g);
   const size_t bytes = (size_t)face * 6 * sizeof(double2);
   double2* d = nullptr;
-  CU(cudaMalloc(&d, 2 * bytes));
+  CU(dev_alloc(ctx, &d, 2 * bytes));
   struct Free
   {
     void* p;

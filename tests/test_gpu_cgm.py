@@ -104,7 +104,8 @@ def test_cgm_window_lengths(cuda_device, graph_iters, precision, niter):
 @pytest.mark.parametrize("precision", ["single", "half", "double"])
 def test_a_window_keeps_no_memory(cuda_device, precision):
     """After a call a window of eight iterations holds what one of a single iteration does: the residuals lie in
-    fields that are idle meanwhile, and what FP64 needs beyond them is given back (64 MiB at most are kept)."""
+    fields that are idle meanwhile.  FP64 needs four fields beyond them, and keeps them while they are a 64th of
+    what is free at most."""
     import torch
     T, L = 24, 16  # FP64: 18.9 MB a field, seven besides the running one
     src = torch.from_numpy(wl.random_spinor(T * L ** 3, 47)).to("cuda:0")
@@ -120,7 +121,10 @@ def test_a_window_keeps_no_memory(cuda_device, precision):
             lat.inv_tmQ2_cgm(0.15, [0.1, 0.5], src, 100000, [1e-16, 1e-16], precision=precision, out=out)
             used.append(free0 - torch.cuda.mem_get_info()[0])
     slack = 16 << 20  # the graphs' own memory
-    assert used[0] <= used[1] + slack, used
+    more = 0
+    if precision == "double" and 64 * 4 * T * L ** 3 * 192 <= torch.cuda.mem_get_info()[0]:
+        more = 4 * T * L ** 3 * 192
+    assert used[0] <= used[1] + more + slack, used
 
 
 @pytest.mark.parametrize("precision", ["single", "double"])
