@@ -433,7 +433,7 @@ tms_status tms_apply_tmclovQ(tms_ctx* ctx, double kappa, int has_anis, double an
   TRY(check_clover(ctx));
   TRY(check_params(ctx, kappa, mu));
   const size_t bytes = (size_t)ctx->g.V * 24 * sizeof(double);
-  const bool planes = ctx->g.V > AOS_CLOVER_SITES || !ctx->small_lattice;
+  const bool planes = ctx->g.V > AOS_CLOVER_Q_SITES || !ctx->small_lattice;
   OpBuffers b;
   TRY(op_begin(ctx, in, out, bytes, planes ? OP_PLANES : OP_GATHER, b));
   const OpParams prm{kappa, mu, has_anis ? anis : 1.0};

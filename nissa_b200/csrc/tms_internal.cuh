@@ -354,7 +354,9 @@ namespace tms_int
   // 4.08 / 2.85, 5.09 / 4.66 (20736: 5.68 / 5.96); FP16 3.47 / 3.23, 3.14 / 2.85,
   // 3.94 / 4.53.  (The e/o solvers of these sizes run in one launch instead where
   // they can, tms_cg_small.cuh: the rule is left to the full-lattice solvers, the
-  // FP64 steps around a solve, and other devices' residency.)
+  // FP64 steps around a solve, and other devices' residency.  So FP32's line stays
+  // where the one launch ends, although its e/o solves still gain at 16800 sites:
+  // full-lattice launches between the two were not measured.)
   constexpr int HOP_DP_SITES_MAX[3] = {6144, 9472, 6144};
 
   template <int P, int LF, class Epi, class Fin = NoFin>
@@ -475,16 +477,18 @@ namespace tms_int
   inline LinkT<LINK_H16_12> links16h(tms_ctx* c) { return LinkT<LINK_H16_12>{c->U16h, (int)c->g.Vh}; }
 
   // ------------------------------------------- operators in the caller's layout
-  // Output sites per hop up to which an operator of several hops works on the
-  // caller's arrays directly; the others convert to planes and back around hops
-  // on planes.  (A single hop, tms_hop_eo or tms_apply_tmQ, is direct at every
-  // size: 32^3x64 hop 424 us, 440 with the conversions.)  Whole calls, direct /
-  // on planes: K^2 at 16800 sites 63.9 / 71.2 us, 20736 72.2 / 79.4, 36864
-  // 91.2 / 87.4, 331776 547 / 459; twisted-clover K^2 at 4096 45.7 / 67.5, 16800
-  // 68.6 / 73.2, 20736 84.5 / 81.8.  The directions' products are spread over a
+  // Output sites per hop up to which an operator works on the caller's arrays
+  // directly; the others convert to planes and back around hops on planes.  (A
+  // single hop, tms_hop_eo or tms_apply_tmQ, is direct at every size: 32^3x64 hop
+  // 425 us, 440 with the conversions.)  The directions' products are spread over a
   // block, so nothing of a neighbour is reused through L1, which costs the more
-  // the more sites there are to hide latencies.
-  constexpr int64_t AOS_KERN_SITES = 25000, AOS_Q2_SITES = 60000, AOS_CLOVER_SITES = 18000;
+  // the more sites there are to hide latencies.  Whole calls, direct / on planes,
+  // in us:
+  //   K^2 (sites of a parity)        17280 50 / 58, 20736 59 / 63, 32928 77 / 68, 40960 88 / 92, 57344 115 / 104
+  //   Q^2 (all sites)                16000 37 / 41, 34560 51 / 47, 41472 58 / 58, 65856 75 / 70, 186624 174 / 152
+  //   twisted-clover K^2 (a parity)  8000 41 / 54, 17280 61 / 64, 20736 76 / 71, 32928 118 / 87
+  //   twisted-clover Q (all sites)   16000 30 / 37, 34560 40 / 41, 41472 46 / 49, 65856 72 / 59
+  constexpr int64_t AOS_KERN_SITES = 25000, AOS_Q2_SITES = 30000, AOS_CLOVER_SITES = 18000, AOS_CLOVER_Q_SITES = 45000;
 
   // one hop from `in` to epi.out, both in the caller's layout: e/o order of
   // parity par_out, or (FULL) lx order; the parameters travel with the launch
